@@ -25,7 +25,14 @@
 // its quotient (max - upwind) / (dt flxIn / hProv + 1e-10) divides
 // rounding-level differences by the regulariser, so any other rounding of the
 // chain moves the step by far more than its own rounding.
+//
+// The FP64 pipe bounds these kernels (82-84% busy with every product and sum on
+// it, the issue slots 10-24%), so the products run on the integer pipe
+// (softmul.cuh, the same rounding bit for bit) and only the sums on the FP64
+// pipe.  Level-6 sphere, 60 levels x 3 tracers, per launch: oc_edges 1384 ->
+// 651 us (FP64 65% busy, integer 63%), oc_cells 659 -> 453, oc_final 484 -> 363.
 #include "rk4.cuh"
+#include "softmul.cuh"
 
 namespace mpaso {
 namespace {
@@ -72,6 +79,14 @@ __global__ void k_oc_prep(DMesh m, int L, const double *u, const double *h, cons
   hpi[i] = 1.0 / hp;
 }
 
+// Rare work of K1, called so that warps without it skip it: inlined, it becomes
+// predicated instructions, which occupy the FP64 pipe all the same (11 a
+// thread beside the 36 sums of three tracers).
+__device__ __noinline__ double masked_weight(double f, int mask) { return f * (double)mask; }
+__device__ __noinline__ double add_centred_flux(double flx, double dv, double f, double t1, double t2) {
+  return flx + (dv * 0.5) * f * (t1 + t2);
+}
+
 // K1: per edge-level, for every tracer, the low-order flux LO
 // (solve.cc:106-116), the high-order flux corrected for FCT, A = HO - LO
 // (solve.cc:143-165, 216-229), and the del2 flux DF = hE (tr2 - tr1) rho
@@ -92,10 +107,12 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
     const int mask = m.hoMask[(int64_t)e * m.fctLev + k];
     // wgtTmp = f mask (solve.cc:145): for a mask of 1 f itself, for 0 the zero
     // with f's sign, on the integer pipe (other masks: the product)
-    const double wgt = mask == 1 ? f : mask == 0 ? bitsd(dbits(f) & kSignBit) : f * (double)mask;
+    const double wgt = mask == 1 ? f : mask == 0 ? bitsd(dbits(f) & kSignBit) : masked_weight(f, mask);
     // sgnTmp = sign(f) picks the factor coef1 + coef3 sgn; where f = 0 the
     // weight wgt is a zero and so is every weightFactor, whichever is picked
     const bool neg = dlt0(f);
+    uint32_t badw = 0;
+    const SoftFactor fw = soft_factor(wgt, badw);
     double flx[T];
 #pragma unroll
     for (int t = 0; t < T; ++t) flx[t] = 0.0;
@@ -104,27 +121,41 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
     for (int a = 0; a < na; ++a) {
       const int64_t sa = (int64_t)a * m.nE + e;
       const int cell = m.advCells[sa];
-      const double2 cf = st.cpm1[sa];
-      const double wf = wgt * (neg ? cf.y : cf.x);  // weightFactor (solve.cc:155)
+      const double2 cf2 = st.cpm1[sa];
+      const double cf = neg ? cf2.y : cf2.x;
       const double *tr = S.tr_in + ((int64_t)cell * L + k) * T;
+      // weightFactor wf = wgt cf (solve.cc:155), then tr wf for every tracer
+      uint32_t bad = badw;
+      const SoftFactor wf = soft_factor(soft_mul(cf, fw, bad), bad);
+      double p[T];
 #pragma unroll
-      for (int t = 0; t < T; ++t) flx[t] += tr[t] * wf;
+      for (int t = 0; t < T; ++t) p[t] = soft_mul(tr[t], wf, bad);
+      if (bad) {
+        const double wx = product_outside(wgt, cf);
+#pragma unroll
+        for (int t = 0; t < T; ++t) p[t] = product_outside(tr[t], wx);
+      }
+#pragma unroll
+      for (int t = 0; t < T; ++t) flx[t] += p[t];
     }
     const double dv = m.dvEdge[e];
     // LO = dv (max(0, f) tr1 + min(0, f) tr2): one of the two products is a zero
     const bool up1 = dgt0(f);
     // tracerWeight of solve.cc:222-223 is a zero on edges whose high-order mask
     // is set (their high-order flux gains nothing); on the others the centred
-    // flux, with ((mask + 1) & 1) = 1.  A branch, not a select: the mask is set
-    // almost everywhere, so warps skip this work instead of issuing it
+    // flux, with ((mask + 1) & 1) = 1
     if (!mask) {
-      const double tw = (dv * 0.5) * f;
 #pragma unroll
-      for (int t = 0; t < T; ++t) flx[t] = flx[t] + tw * (t1[t] + t2[t]);
+      for (int t = 0; t < T; ++t) flx[t] = add_centred_flux(flx[t], dv, f, t1[t], t2[t]);
     }
+    uint32_t badl = 0;
+    const SoftFactor ff = soft_factor(f, badl), fdv = soft_factor(dv, badl);
 #pragma unroll
     for (int t = 0; t < T; ++t) {
-      const double lo = dv * (f * (up1 ? t1[t] : t2[t]));
+      const double x = up1 ? t1[t] : t2[t];
+      uint32_t bad = badl;
+      double lo = soft_mul(soft_mul(x, ff, bad), fdv, bad);
+      if (bad) lo = product_outside(dv, product_outside(f, x));
       S.LO[i * T + t] = lo;
       S.A[i * T + t] = flx[t] - lo;
     }
@@ -132,8 +163,16 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
   if (S.hmix) {
     const double hr = S.hE[i];
     const double rho = st.kd[e];
+    uint32_t badm = 0;
+    const SoftFactor fh = soft_factor(hr, badm), fr = soft_factor(rho, badm);
 #pragma unroll
-    for (int t = 0; t < T; ++t) S.DF[i * T + t] = hr * (t2[t] - t1[t]) * rho;
+    for (int t = 0; t < T; ++t) {
+      const double d = t2[t] - t1[t];
+      uint32_t bad = badm;
+      double x = soft_mul(soft_mul(d, fh, bad), fr, bad);
+      if (bad) x = product_outside(product_outside(hr, d), rho);
+      S.DF[i * T + t] = x;
+    }
   }
 }
 
@@ -158,6 +197,8 @@ __global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
   const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
   const int n = m.nEoC[c];
   const double invAreaCell1 = m.invAreaCell[c];  // 1 / areaCell
+  uint32_t bada = 0;
+  const SoftFactor fa = soft_factor(invAreaCell1, bada);
   double trc[T], mx[T], mn[T], td[T], fi[T], fo[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) {
@@ -175,8 +216,12 @@ __global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
       mx[t] = dmax(mx[t], x);
       mn[t] = dmin(mn[t], x);
       if (ok) {
-        td[t] += dflip(invAreaCell1 * S.LO[ie0 + t], sm);
-        const double ax = dflip(invAreaCell1 * S.A[ie0 + t], sm);
+        const double lo = S.LO[ie0 + t], ho = S.A[ie0 + t];
+        uint32_t bad = bada;
+        double pl = soft_mul(lo, fa, bad), pa = soft_mul(ho, fa, bad);
+        if (bad) pl = product_outside(invAreaCell1, lo), pa = product_outside(invAreaCell1, ho);
+        td[t] += dflip(pl, sm);
+        const double ax = dflip(pa, sm);
         // flxIn += max(0, ax), flxOut += min(0, ax): one add into the sum the
         // sign selects (integer-pipe selects; a zero ax changes neither sum,
         // so none is kept), instead of an add in each of two divergent branches
@@ -191,9 +236,9 @@ __global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
   const double eps = 1.e-10;
 #pragma unroll
   for (int t = 0; t < T; ++t) {
-    const double up = (trc[t] * h + dt * td[t]) * hpi;  // tracerUpwindNew
-    const double mxn = up + dt * fi[t] * hpi;            // tracerMaxNew
-    const double mnn = up + dt * fo[t] * hpi;            // tracerMinNew
+    const double up = mul_int(mul_int(trc[t], h) + mul_int(td[t], dt), hpi);  // tracerUpwindNew
+    const double mxn = up + mul_int(mul_int(fi[t], dt), hpi);                 // tracerMaxNew
+    const double mnn = up + mul_int(mul_int(fo[t], dt), hpi);                 // tracerMinNew
     const double rp = clamp_quotient(mx[t] - up, (mxn - up) + eps);
     const double rm = clamp_quotient(up - mn[t], (up - mnn) + eps);
     S.R2[i * T + t] = make_double2(rp, rm);
@@ -214,6 +259,8 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
   const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
   const int n = m.nEoC[c];
   const double invAreaCell1 = m.invAreaCell[c];
+  uint32_t bada = 0;
+  const SoftFactor fa = soft_factor(invAreaCell1, bada);
   double td[T];
   double2 own[T];
 #pragma unroll
@@ -239,8 +286,13 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
         // max(0, A) / min(0, A) terms give
         const bool pos = dgt0(a);
         const double rmin = pos ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
-        const double hl = (dgt0(a) || dlt0(a) ? a : 0.0) * rmin;
-        td[t] += dflip(invAreaCell1 * hl, sm);
+        // (a zero factor -- local extrema -- makes the flux the zero, the other 1)
+        const bool some = dgt0(rmin);
+        const double a0 = some && (pos || dlt0(a)) ? a : 0.0, r0 = some ? rmin : 1.0;
+        uint32_t bad = bada;
+        double x = soft_mul(soft_mul(a0, soft_factor(r0, bad), bad), fa, bad);
+        if (bad) x = product_outside(invAreaCell1, product_outside(a0, r0));
+        td[t] += dflip(x, sm);
       }
     });
   }
@@ -251,7 +303,13 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
       const long long sm = sign_mask(m.eocSign[s]);
       const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;
 #pragma unroll
-      for (int t = 0; t < T; ++t) td[t] -= dflip(S.DF[ie0 + t] * invAreaCell1, sm);
+      for (int t = 0; t < T; ++t) {
+        const double d = S.DF[ie0 + t];
+        uint32_t bad = bada;
+        double x = soft_mul(d, fa, bad);
+        if (bad) x = product_outside(d, invAreaCell1);
+        td[t] -= dflip(x, sm);
+      }
     });
   }
 #pragma unroll
@@ -260,15 +318,15 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
     const double cur = S.tr_prev[j];
     switch (S.stage) {  // tracersNew += w tend; tracersPrev = tracers + w_sub tend
       case 0:
-        S.trh_acc[j] = cur + S.w_acc * td[t];
-        S.tr_out[j] = cur + S.w_sub * td[t];
+        S.trh_acc[j] = cur + mul_int(td[t], S.w_acc);
+        S.tr_out[j] = cur + mul_int(td[t], S.w_sub);
         break;
       case 3:
-        S.tr_new[j] = S.trh_acc[j] + S.w_acc * td[t];
+        S.tr_new[j] = S.trh_acc[j] + mul_int(td[t], S.w_acc);
         break;
       default:
-        S.trh_acc[j] = S.trh_acc[j] + S.w_acc * td[t];
-        S.tr_out[j] = cur + S.w_sub * td[t];
+        S.trh_acc[j] = S.trh_acc[j] + mul_int(td[t], S.w_acc);
+        S.tr_out[j] = cur + mul_int(td[t], S.w_sub);
     }
   }
 }

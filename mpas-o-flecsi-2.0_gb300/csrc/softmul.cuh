@@ -1,0 +1,97 @@
+// IEEE double products on the integer pipe.
+//
+// GB300 issues one FP64 warp instruction per SM every 16 cycles while the four
+// schedulers could issue 64 others in that time, so a kernel whose FP64
+// instructions are half products and half sums (the reference's rounding
+// allows no fused multiply-add) leaves most issue slots idle.  soft_mul forms
+// the correctly rounded (nearest, ties to even) product of two doubles from
+// four 32 x 32 -> 64 bit integer products, equal bit for bit to the hardware
+// product (1.3e9 random and special pairs), and leaves the FP64 pipe to the
+// sums.  Measured in SM cycles per warp instruction: DMUL and DADD 19.1 each,
+// soft_mul 12.0 alone (9.9 without the in-line zero), soft_mul with a DADD on
+// its result 19.2 against DMUL + DADD 38.2: the products cost nothing beside
+// the sums.  The ALU pipe bounds it; moving its shifts to multiplications
+// (14.7) or its additions to multiply-adds (13.1) was slower.
+//
+// Both factors must have an exponent in [kSoftLo, kSoftLo + 512) (magnitudes
+// 2^-256 .. 2^256, so no product overflows or underflows); others -- subnormals,
+// infinities, NaN, a zero second factor -- set a bit of `bad` and the caller
+// takes product_outside() instead.  A zero first factor is common (tracer
+// plateaus, still water) and gives +0 in line: a branch that single lanes of
+// most warps take would make the warp issue the sums behind it twice, once
+// for each side.  The sign of such a zero is not kept; the sums it enters
+// start from +0 and cannot tell.
+#pragma once
+
+#include <cstdint>
+
+#include "device.cuh"
+
+namespace mpaso {
+
+constexpr uint32_t kSoftLo = 767u << 20;       // lowest exponent, at its place in the high word
+constexpr uint32_t kSoftRange = 0x60000000u;   // set by exponents outside the window
+
+// A factor prepared once for several products: significand shifted up by 10
+// bits (so the cross products cannot overflow 64 bits), sign and exponent
+// relative to kSoftLo.
+struct SoftFactor {
+  uint32_t h, l, x;
+};
+
+// `x` of a factor: sign and exponent fields relative to the window's start.
+// An exponent outside it borrows into or reaches bits 29 and 30.
+__device__ __forceinline__ uint32_t soft_exp(uint32_t hi) { return (hi & 0xfff00000u) - kSoftLo; }
+
+__device__ __forceinline__ SoftFactor soft_factor(double b, uint32_t &bad) {
+  const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
+  SoftFactor f;
+  f.h = (__funnelshift_l(lo, hi, 10) & 0x3fffffffu) | 0x40000000u;
+  f.l = lo << 10;
+  f.x = soft_exp(hi);
+  bad |= f.x & kSoftRange;
+  return f;
+}
+
+__device__ __forceinline__ double soft_mul(double a, const SoftFactor &f, uint32_t &bad) {
+  const uint32_t hi = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
+  const uint32_t x = soft_exp(hi);
+  const bool zero = ((hi & 0x7fffffffu) | al) == 0;
+  bad |= zero ? 0u : x & kSoftRange;
+  const uint32_t ah = (hi & 0xfffffu) | 0x100000u;
+  // P = a f 2^10 = top 2^64 + lo(t2) 2^32 + lo(t0), in [2^114, 2^116)
+  const uint64_t t0 = (uint64_t)al * f.l;
+  const uint64_t t1 = (uint64_t)ah * f.l + (t0 >> 32);
+  const uint64_t t2 = (uint64_t)al * f.h + t1;  // < 2^63 + 2^54
+  const uint64_t top = (uint64_t)ah * f.h + (t2 >> 32);
+  const uint32_t th = (uint32_t)(top >> 32), tl = (uint32_t)top, tr = (uint32_t)t2;
+  const uint32_t n = th >> 19;  // 1 where the significands' product is >= 2
+  const uint32_t s = 2 - n;     // brings the leading bit to the implicit bit's place
+  const uint32_t mh = __funnelshift_l(tl, th, s), ml = __funnelshift_l(tr, tl, s), r = tr << s;
+  // round to nearest even: r + 0x7fffffff + (odd | sticky) carries exactly when
+  // the discarded part exceeds a half, or equals it and the result is odd
+  const uint32_t inc = ((ml | min((uint32_t)t0, 1u)) & 1u) + 0x7fffffffu;
+  const uint32_t e = x + f.x + n * 0x100000u + ((2 * 767 - 1023 - 1) << 20);
+  uint32_t oh, ol;
+  asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
+      : "=r"(ol), "=r"(oh)
+      : "r"(r), "r"(inc), "r"(ml), "r"(mh), "r"(e));
+  return __hiloint2double(zero ? 0 : (int)oh, zero ? 0 : (int)ol);
+}
+
+// The product where soft_mul's window does not hold.  A call, not inlined:
+// few warps need it, and the compiler turns a plain branch around an inlined
+// multiplication into a predicated one, which occupies the FP64 pipe for the
+// whole warp even where no lane takes it.
+static __device__ __noinline__ double product_outside(double a, double b) { return a * b; }
+
+// One product on the integer pipe.
+__device__ __forceinline__ double mul_int(double a, double b) {
+  uint32_t bad = 0;
+  const SoftFactor f = soft_factor(b, bad);
+  double r = soft_mul(a, f, bad);
+  if (bad) r = product_outside(a, b);
+  return r;
+}
+
+}  // namespace mpaso
