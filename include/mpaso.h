@@ -293,7 +293,9 @@ int mpaso_state_device_bytes(mpaso_state s, int64_t *bytes);
  * of the second, the limiter into a kernel of its own).  Results do not
  * depend on the threads per block, the L2 choice, the launch overlap or the
  * schedule; the other variants may
- * differ in the last bits.  No counterpart in the reference (its tasks have
+ * differ in the last bits.  A state reports 256 threads and no overlap until a
+ * configuration is set or tuned; until then its launches choose both by the
+ * mesh's size.  No counterpart in the reference (its tasks have
  * no device launch shape).  Setting it drops any captured step graph; a
  * persisting L2 reservation is per device context, so at most one state per
  * device should use config[9] != 0, and destroying it releases the

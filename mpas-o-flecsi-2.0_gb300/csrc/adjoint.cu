@@ -136,7 +136,10 @@ void free_adjoint(SwState &s) {
 
 namespace {
 
-constexpr int TPB = 256;
+constexpr int TPB = 256;  // bound of the kernels' registers
+// Threads per block launched: small ones spread a small mesh over all SMs (level
+// 5, (h, u), 40 steps, forward + vjp with 256 / 128 / 64: 4.98 / 4.81 / 4.77 ms).
+constexpr int TPL = 64;
 
 struct AdjArgs {
   const double *u, *h;                        // stage state
@@ -177,7 +180,7 @@ struct TrArgs {
 
 // Edge quantities of a stage state that B1 gathers: F = u he, pve from the taped
 // vertex pv, and P = lk_u pve (lk_u: the stage tendency's cotangent).
-__device__ __forceinline__ void prep_edge(const DMesh &m, const AdjArgs &a, int L, int e, int k, int64_t i,
+__device__ __forceinline__ void prep_edge(const DMesh &m, const AdjArgs &a, Lev L, int e, int k, int64_t i,
                                           const double *u, const double *h, const double *pv, double lk) {
   const int2 c = m.coe[e];
   const int2 v = m.voe[e];
@@ -189,11 +192,12 @@ __device__ __forceinline__ void prep_edge(const DMesh &m, const AdjArgs &a, int 
 
 // PREP (edges): the above for the first stage reversed in a segment (later
 // stages get it from the B3 before them).
-__global__ void __launch_bounds__(TPB) k_adj_prep(DMesh m, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_prep(DMesh m, AdjArgs a, Lev L) {
   stage_prologue();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   prep_edge(m, a, L, e, k, i, a.u, a.h, a.pv, a.lk_u[i]);
 }
 
@@ -202,9 +206,10 @@ __global__ void __launch_bounds__(TPB) k_adj_prep(DMesh m, AdjArgs a, int L) {
 // `tr`: the tracer part's thickness-flux and edge-thickness cotangents lFt,
 // lhet of this edge (from TB) are added.
 template <int NW>
-__device__ __forceinline__ void b1_item(const DMesh &m, const AdjArgs &a, int L, int64_t i, bool tr, double lFt,
+__device__ __forceinline__ void b1_item(const DMesh &m, const AdjArgs &a, Lev L, int64_t i, bool tr, double lFt,
                                         double lhet) {
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   // S1 = sum_j W_j F_j comes from the forward's tape (4 x its W/8 . 2F sum, exact)
   const double s1 = 4.0 * a.s1[i];
   double t1 = 0.0, t2 = 0.0;
@@ -235,7 +240,7 @@ __device__ __forceinline__ void b1_item(const DMesh &m, const AdjArgs &a, int L,
 }
 
 template <int NW>
-__global__ void __launch_bounds__(TPB) k_adj_b1(DMesh m, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_b1(DMesh m, AdjArgs a, Lev L) {
   stage_prologue();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
@@ -245,9 +250,10 @@ __global__ void __launch_bounds__(TPB) k_adj_b1(DMesh m, AdjArgs a, int L) {
 
 // B2 (cells + vertices): gradient terms, h_e -> h, pv -> (circ, hs).
 // `muh`: the tracer part's thickness cotangent of this cell (0 without tracers).
-__device__ __forceinline__ void b2_cell_item(const DMesh &m, const AdjArgs &a, int L, int64_t i, double muh) {
+__device__ __forceinline__ void b2_cell_item(const DMesh &m, const AdjArgs &a, Lev L, int64_t i, double muh) {
   {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     double G = 0.0, sl = 0.0;
     auto slot = [&](int j, bool ok) {
       const int64_t s = (int64_t)j * m.nC + c;
@@ -266,8 +272,9 @@ __device__ __forceinline__ void b2_cell_item(const DMesh &m, const AdjArgs &a, i
   }
 }
 
-__device__ __forceinline__ void b2_vertex_item(const DMesh &m, const AdjArgs &a, int L, int64_t i) {
-  const int v = (int)(i / L), k = (int)(i - (int64_t)v * L);
+__device__ __forceinline__ void b2_vertex_item(const DMesh &m, const AdjArgs &a, Lev L, int64_t i) {
+  int v, k;
+  L.split(i, v, k);
   double lpv = 0.0, lvort = 0.0;
 #pragma unroll
   for (int j = 0; j < kVertexDegree; ++j) {
@@ -285,7 +292,7 @@ __device__ __forceinline__ void b2_vertex_item(const DMesh &m, const AdjArgs &a,
   a.lhs[i] = -lpv * a.pv[i] * rh;
 }
 
-__global__ void __launch_bounds__(TPB) k_adj_b2(DMesh m, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_b2(DMesh m, AdjArgs a, Lev L) {
   stage_prologue();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
@@ -326,8 +333,9 @@ __device__ __forceinline__ double combine(int rk, double dt, int64_t i, double m
 
 // B3 (cells + edges): thickness through kites; u through circulation, KE and
 // divergence; then the RK combination.
-__device__ __forceinline__ void b3_cell_item(const DMesh &m, const AdjArgs &a, int L, int64_t i) {
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+__device__ __forceinline__ void b3_cell_item(const DMesh &m, const AdjArgs &a, Lev L, int64_t i) {
+  int c, k;
+  L.split(i, c, k);
   double mh = a.mu_h[i];
   for (int j = 0; j < m.maxEoC; ++j) {
     const int64_t s = (int64_t)j * m.nC + c;
@@ -336,8 +344,9 @@ __device__ __forceinline__ void b3_cell_item(const DMesh &m, const AdjArgs &a, i
   combine(a.rk, a.dt, i, mh, a.lam_h, a.acc_h, a.lk_h);
 }
 
-__device__ __forceinline__ void b3_edge_item(const DMesh &m, const DStat &st, const AdjArgs &a, int L, int64_t i) {
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+__device__ __forceinline__ void b3_edge_item(const DMesh &m, const DStat &st, const AdjArgs &a, Lev L, int64_t i) {
+  int e, k;
+  L.split(i, e, k);
   const int2 c = m.coe[e];
   const int2 v = m.voe[e];
   const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
@@ -351,7 +360,7 @@ __device__ __forceinline__ void b3_edge_item(const DMesh &m, const DStat &st, co
   if (a.prep) prep_edge(m, a, L, e, k, i, a.un, a.hn, a.pvn, lk);
 }
 
-__global__ void __launch_bounds__(TPB) k_adj_b3(DMesh m, DStat st, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_b3(DMesh m, DStat st, AdjArgs a, Lev L) {
   stage_prologue();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
@@ -392,10 +401,11 @@ template <int NL> __device__ __forceinline__ double lane_sum(double v) {
 // slots; the bounds merge as (value, slot) with the lower slot (the cell
 // itself first) winning ties, which is the reference's sequential max / min.
 template <int NL, int NC>
-__device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, int L, int64_t g) {
+__device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L, int64_t g) {
   const int lane = (int)(g & (NL - 1));
   const int64_t i = g / NL;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const int n = m.nEoC[c], T = a.T;
   const double hin = a.h[i], hpi = a.hpi[i];
   const double dtia = a.dt * m.invAreaCell[c];
@@ -490,7 +500,7 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, int L
 }
 
 template <int NL, int NC>
-__global__ void __launch_bounds__(TPB) k_adj_tr_a(DMesh m, TrArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_tr_a(DMesh m, TrArgs a, Lev L) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (g / NL >= (int64_t)m.nC * L) return;  // whole groups: all lanes of a live cell stay
   tr_a_item<NL, NC>(m, a, L, g);
@@ -500,7 +510,7 @@ __global__ void __launch_bounds__(TPB) k_adj_tr_a(DMesh m, TrArgs a, int L) {
 // forward, same segment): TA of a cell-level reads, of what B3 writes, only
 // the thickness-tendency cotangent of its own cell, so one thread does both.
 template <int NC>
-__global__ void __launch_bounds__(TPB) k_adj_b3_tra(DMesh m, DStat st, AdjArgs a, TrArgs tn, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_b3_tra(DMesh m, DStat st, AdjArgs a, TrArgs tn, Lev L) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (i < nCL) {
@@ -524,9 +534,11 @@ __global__ void __launch_bounds__(TPB) k_adj_b3_tra(DMesh m, DStat st, AdjArgs a
 // tracer the parts for cells(e) go to p12 and lambda_HO F, split by the sign
 // of F, to lho (TC gathers them); per edge the thickness-flux and
 // edge-thickness cotangents summed over tracers go to lFt / lhet (B1 adds them).
-__device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, int L, int64_t i, double &lF_out,
+__device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, Lev L, int64_t i, double &lF_out,
                                           double &lhe_out) {
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L), T = a.T;
+  int e, k;
+  L.split(i, e, k);
+  const int T = a.T;
   const int2 c = m.coe[e];
   const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
   const double he = a.ocean ? a.hEx[i] : 0.5 * (a.h[i1] + a.h[i2]);
@@ -597,7 +609,7 @@ __device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, int L
   lF_out = lF, lhe_out = lhe;
 }
 
-__global__ void __launch_bounds__(TPB) k_adj_tr_b(DMesh m, TrArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_tr_b(DMesh m, TrArgs a, Lev L) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
   double lF, lhe;
@@ -615,10 +627,11 @@ __global__ void __launch_bounds__(TPB) k_adj_tr_b(DMesh m, TrArgs a, int L) {
 // cell split the gathers and sum by shuffles.
 // Returns true on the lane that holds the cell's thickness cotangent mh_out.
 template <int NL>
-__device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, int L, int64_t g, double &mh_out) {
+__device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L, int64_t g, double &mh_out) {
   const int lane = (int)(g & (NL - 1));
   const int64_t i = g / NL;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const int n = m.nEoC[c], T = a.T;
   const double hinv = a.ocean ? 1.0 : rcp_nr(a.h[i]), inva = m.invAreaCell[c];
   double mh = a.fct && !a.ocean ? a.muh_t[i] : 0.0;
@@ -677,7 +690,7 @@ __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, int L
 }
 
 template <int NL>
-__global__ void __launch_bounds__(TPB) k_adj_tr_c(DMesh m, TrArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_tr_c(DMesh m, TrArgs a, Lev L) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (g / NL >= (int64_t)m.nC * L) return;  // whole groups: all lanes of a live cell stay
   double mh;
@@ -687,7 +700,7 @@ __global__ void __launch_bounds__(TPB) k_adj_tr_c(DMesh m, TrArgs a, int L) {
 // The sw app with tracers, fused by item: TB and B1 of one edge-level in one
 // thread (the tracer part's flux cotangents pass in registers) ...
 template <int NW>
-__global__ void __launch_bounds__(TPB) k_adj_trb_b1(DMesh m, TrArgs t, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_trb_b1(DMesh m, TrArgs t, AdjArgs a, Lev L) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
   double lF, lhe;
@@ -699,7 +712,7 @@ __global__ void __launch_bounds__(TPB) k_adj_trb_b1(DMesh m, TrArgs t, AdjArgs a
 // the cell part of B2 with the thickness cotangent in hand; the threads past
 // the cells do B2's vertices.
 template <int NL>
-__global__ void __launch_bounds__(TPB) k_adj_trc_b2(DMesh m, TrArgs t, AdjArgs a, int L) {
+__global__ void __launch_bounds__(TPB) k_adj_trc_b2(DMesh m, TrArgs t, AdjArgs a, Lev L) {
   int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (g < nCL * NL) {
@@ -734,7 +747,7 @@ __global__ void k_adj_q_convert(int64_t nCL, int T, const double *h, const doubl
 }
 
 // lk_q = c lam_q and g = lk_q / areaCell
-__global__ void k_adj_init_q(DMesh m, int L, int T, const double *lam, double *lk, double *g, double c) {
+__global__ void k_adj_init_q(DMesh m, Lev L, int T, const double *lam, double *lk, double *g, double c) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L * T) return;
   const double l = c * lam[i];
@@ -872,15 +885,15 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
   // plain stream order: programmatic dependent launch made this 25% slower (measured)
   const bool pdl = false;
   const bool ocean = s.p.app == MPASO_APP_OCEAN;
-  if (first && !ocean) launch_pdl(k_adj_prep, nE, TPB, pdl, st, m, a, L);
+  if (first && !ocean) launch_pdl(k_adj_prep, nE, TPL, pdl, st, m, a, L);
   if (A.tr) {
     const TrArgs t = tr_args(s, A, rk, j);
     constexpr int NLA = 1, NLC = 2;  // lanes per cell (measured best at level 6)
     if (t.fct && !tra_done) {
       if (m.maxEoC <= 6)
-        launch_pdl(k_adj_tr_a<NLA, 6>, nC * NLA, TPB, pdl, st, m, t, L);
+        launch_pdl(k_adj_tr_a<NLA, 6>, nC * NLA, TPL, pdl, st, m, t, L);
       else
-        launch_pdl(k_adj_tr_a<NLA, 0>, nC * NLA, TPB, pdl, st, m, t, L);
+        launch_pdl(k_adj_tr_a<NLA, 0>, nC * NLA, TPL, pdl, st, m, t, L);
     }
     // two lanes per cell-level hide gather latency on small meshes; with a
     // million cell-levels or more there is parallelism enough, and the
@@ -889,37 +902,37 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
     if (!ocean) {
       // sw: TB with B1 and TC with B2 as two fused launches, then B3
       if (m.maxEoE == 10)
-        launch_pdl(k_adj_trb_b1<10>, nE, TPB, pdl, st, m, t, a, L);
+        launch_pdl(k_adj_trb_b1<10>, nE, TPL, pdl, st, m, t, a, L);
       else
-        launch_pdl(k_adj_trb_b1<0>, nE, TPB, pdl, st, m, t, a, L);
+        launch_pdl(k_adj_trb_b1<0>, nE, TPL, pdl, st, m, t, a, L);
       if (one_lane)
-        launch_pdl(k_adj_trc_b2<1>, nC + nV, TPB, pdl, st, m, t, a, L);
+        launch_pdl(k_adj_trc_b2<1>, nC + nV, TPL, pdl, st, m, t, a, L);
       else
-        launch_pdl(k_adj_trc_b2<NLC>, nC * NLC + nV, TPB, pdl, st, m, t, a, L);
+        launch_pdl(k_adj_trc_b2<NLC>, nC * NLC + nV, TPL, pdl, st, m, t, a, L);
       if (t.fct && prep_next) {  // with TA of the next reversed stage (slot j - 1)
         const TrArgs tn = tr_args(s, A, rk > 0 ? rk - 1 : 3, j - 1);
         if (m.maxEoC <= 6)
-          launch_pdl(k_adj_b3_tra<6>, nC + nE, TPB, pdl, st, m, s.st, a, tn, L);
+          launch_pdl(k_adj_b3_tra<6>, nC + nE, TPL, pdl, st, m, s.st, a, tn, L);
         else
-          launch_pdl(k_adj_b3_tra<0>, nC + nE, TPB, pdl, st, m, s.st, a, tn, L);
+          launch_pdl(k_adj_b3_tra<0>, nC + nE, TPL, pdl, st, m, s.st, a, tn, L);
         return true;
       }
-      launch_pdl(k_adj_b3, nC + nE, TPB, pdl, st, m, s.st, a, L);
+      launch_pdl(k_adj_b3, nC + nE, TPL, pdl, st, m, s.st, a, L);
       return false;
     }
-    launch_pdl(k_adj_tr_b, nE, TPB, pdl, st, m, t, L);
+    launch_pdl(k_adj_tr_b, nE, TPL, pdl, st, m, t, L);
     if (one_lane)
-      launch_pdl(k_adj_tr_c<1>, nC, TPB, pdl, st, m, t, L);
+      launch_pdl(k_adj_tr_c<1>, nC, TPL, pdl, st, m, t, L);
     else
-      launch_pdl(k_adj_tr_c<NLC>, nC * NLC, TPB, pdl, st, m, t, L);
+      launch_pdl(k_adj_tr_c<NLC>, nC * NLC, TPL, pdl, st, m, t, L);
   }
   if (ocean) return false;  // the ocean's h and u are prescribed: nothing more to reverse
   if (m.maxEoE == 10)
-    launch_pdl(k_adj_b1<10>, nE, TPB, pdl, st, m, a, L);
+    launch_pdl(k_adj_b1<10>, nE, TPL, pdl, st, m, a, L);
   else
-    launch_pdl(k_adj_b1<0>, nE, TPB, pdl, st, m, a, L);
-  launch_pdl(k_adj_b2, nC + nV, TPB, pdl, st, m, a, L);
-  launch_pdl(k_adj_b3, nC + nE, TPB, pdl, st, m, s.st, a, L);
+    launch_pdl(k_adj_b1<0>, nE, TPL, pdl, st, m, a, L);
+  launch_pdl(k_adj_b2, nC + nV, TPL, pdl, st, m, a, L);
+  launch_pdl(k_adj_b3, nC + nE, TPL, pdl, st, m, s.st, a, L);
   return false;
 }
 

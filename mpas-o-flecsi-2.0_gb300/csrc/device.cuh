@@ -32,6 +32,26 @@ constexpr int kMaxTracers = 8;
       ::mpaso::fail(MPASO_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Level count of a launch with what splits a flat (entity, level) index without
+// a 64-bit division (a subroutine of some hundred cycles at the head of every
+// kernel): i / L is the high half of i (floor(2^64 / L) + 1), exact for
+// i < 2^64 / L (Granlund and Montgomery 1994).
+struct Lev {
+  int L = 1;
+  uint64_t mul = 0;
+  Lev() = default;
+  __host__ Lev(int l) : L(l) {
+    if (l > 1) mul = ~0ull / (uint64_t)l + 1 + ((~0ull % (uint64_t)l) + 1 == (uint64_t)l ? 1 : 0);
+  }
+  __host__ __device__ operator int() const { return L; }
+  // e = i / L, k = i % L
+  __device__ __forceinline__ void split(int64_t i, int &e, int &k) const {
+    const uint64_t q = __umul64hi((uint64_t)i, mul);
+    e = L == 1 ? (int)i : (int)q;
+    k = (int)i - e * L;
+  }
+};
+
 // Device view of a mesh context (all pointers are device memory).
 struct DMesh {
   int nC, nE, nV;

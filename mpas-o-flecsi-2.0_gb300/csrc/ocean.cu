@@ -351,7 +351,7 @@ template <int T> void ocean_stage_T(SwState &s, const Stage &S, cudaStream_t st)
   const DMesh &m = s.mesh->ctx.d;
   const int L = s.L;
   cudaEvent_t *ev = s.prof_events;
-  const int b0 = s.tune_tpb[0], b1 = s.tune_tpb[1], b2 = s.tune_tpb[2];
+  const int b0 = stage_tpb(s, 0), b1 = stage_tpb(s, 1), b2 = stage_tpb(s, 2);
   if (m.maxAdv == 10 && s.tune_unroll[0])
     k_oc_edges<T, 10><<<blocks_for((int64_t)m.nE * L, b0), b0, 0, st>>>(m, s.st, S, L);
   else

@@ -47,10 +47,11 @@ constexpr int kLanesMaxT = 1;  // variants with 2 or 4 lanes per edge exist up t
 // One edge-level of the pre-pass.  RO: inputs through the read-only path
 // (false inside the persistent kernel).
 template <int T, int NW, bool RO>
-__device__ __forceinline__ void edge_pre_item(const DMesh &m, const DStat &st, const Stage &S, int L, int64_t i) {
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
-  const int2 c = __ldcs(&m.coe[e]);
-  const int2 v = __ldcs(&m.voe[e]);
+__device__ __forceinline__ void edge_pre_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
+  int e, k;
+  L.split(i, e, k);
+  const int2 c = __ldcs(m.coe + (e));
+  const int2 v = __ldcs(m.voe + (e));
   const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
   const double hs = ld_in<RO>(&S.h_in[i1]) + ld_in<RO>(&S.h_in[i2]);  // 2 h_edge
   const double F = ld_in<RO>(&S.u_in[i]) * hs;                         // 2 u h_edge
@@ -61,7 +62,7 @@ __device__ __forceinline__ void edge_pre_item(const DMesh &m, const DStat &st, c
 }
 
 template <int T, int NW, int OC>
-__global__ void MPASO_BOUNDS(OC) k_sw_edge_pre(DMesh m, DStat st, Stage S, int L) {
+__global__ void MPASO_BOUNDS(OC) k_sw_edge_pre(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
   // grid-stride over edge-levels: launched on at most the blocks the SMs hold
   // at once, so the work ends without a partial last wave (measured 37.4 ->
@@ -92,19 +93,20 @@ template <int LANES> __device__ __forceinline__ double lane_total(double x) {
 }
 
 template <int T, int NW, int SPLIT, int LANES = 1>
-__device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const Stage &S, int L, int64_t i) {
+__device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
   const int64_t nEL = (int64_t)m.nE * L;
   if (i < nEL * LANES) {
     const int lane = (int)(i & (LANES - 1));
     i /= LANES;
-    const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+    int e, k;
+    L.split(i, e, k);
     // q = sum_j W_j F_j (pv_e + pv_j) / 2 = (Pv_e sum W/8 F2_j + sum W/8 F2_j Pv_j)
     double s1 = 0.0, s2 = 0.0;
     const int ne = NW > 0 ? NW : m.maxEoE;
 #pragma unroll
     for (int j = lane; j < ne; j += LANES) {
-      const int eo = __ldcs(&m.eoe[(int64_t)j * m.nE + e]);
-      const double w = __ldcs(&st.woe8[(int64_t)j * m.nE + e]);
+      const int eo = __ldcs(m.eoe + ((int64_t)j * m.nE + e));
+      const double w = __ldcs(st.woe8 + ((int64_t)j * m.nE + e));
       const int64_t io = (int64_t)eo * L + k;
       const double2 fg = S.FG[io];
       s1 = fma(w, fg.x, s1);
@@ -114,7 +116,6 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
     s2 = lane_total<LANES>(s2);
     if (lane) return;
     const double q = fma(S.pve[i], s1, s2);
-    if (S.tape_s1) S.tape_s1[i] = s1;
     const int2 c = m.coe[e];
     const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
     // - (ke2 - ke1 + g (h2 + b2 - h1 - b1)) / dc + nu (div2 - div1) / dc, with the
@@ -127,18 +128,15 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
       const int2 v = m.voe[e];
       tend = fma(-st.nuDv[e], S.vort[(int64_t)v.y * L + k] - S.vort[(int64_t)v.x * L + k], tend);
     }
-    const double up = S.u_prev[i];
-    switch (S.stage) {
-      case 0:
-        S.u_out[i] = S.pin_u ? up : fma(S.w_sub, tend, up);
-        S.u_acc[i] = fma(S.w_acc, tend, up);
-        break;
-      case 3:
-        S.u_new[i] = S.pin_u ? up : fma(S.w_acc, tend, S.u_acc[i]);
-        break;
-      default:
-        S.u_out[i] = S.pin_u ? up : fma(S.w_sub, tend, up);
-        S.u_acc[i] = fma(S.w_acc, tend, S.u_acc[i]);
+    // every load before the first store (see the cells below)
+    const double up = S.u_prev[i], acc0 = S.stage == 0 ? up : S.u_acc[i];
+    const double acc = fma(S.w_acc, tend, acc0), out = S.pin_u ? up : fma(S.w_sub, tend, up);
+    if (S.tape_s1) S.tape_s1[i] = s1;
+    if (S.stage == 3) {
+      S.u_new[i] = S.pin_u ? up : acc;
+    } else {
+      S.u_out[i] = out;
+      S.u_acc[i] = acc;
     }
     if constexpr (SPLIT && T > 0)
       edge_tracer_fluxes<T, NW>(m, S, L, e, k, i, i1, i2, S.FG[i].x, h1 + h2, st.dvh, st.cpm2, st.kdh);
@@ -147,40 +145,39 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
   i -= nEL * LANES;
   if (i >= (int64_t)m.nC * L) return;
   constexpr int NC = NW > 0 ? 6 : 0;  // the unrolled variant also unrolls the cell loops
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const int n = m.nEoC[c];
   double tend_h = 0.0;  // sum edgeSign dv F / area, from F2 with the halved weights (0 in pads)
   for_slots<NC>(n, [&](int j, bool) {
     const int64_t s = (int64_t)j * m.nC + c;
     tend_h = fma(st.sdvi[s], S.FG[(int64_t)m.eoc[s] * L + k].x, tend_h);
   });
-  const double hp = S.h_prev[i];
-  switch (S.stage) {
-    case 0:
-      S.h_out[i] = fma(S.w_sub, tend_h, hp);
-      S.h_acc[i] = fma(S.w_acc, tend_h, hp);
-      break;
-    case 3:
-      S.h_new[i] = fma(S.w_acc, tend_h, S.h_acc[i]);
-      break;
-    default:
-      S.h_out[i] = fma(S.w_sub, tend_h, hp);
-      S.h_acc[i] = fma(S.w_acc, tend_h, S.h_acc[i]);
-  }
+  // The stores come last: a load behind a store to memory it might alias waits
+  // for a round trip of its own, and on a mesh too small to fill the GPU those
+  // round trips are most of the kernel.
+  const double hp = S.h_prev[i], acc0 = S.stage == 0 ? hp : S.h_acc[i];
   if constexpr (T > 0) {
     // provisional thickness (apps/ocean/tasks/solve.cc:60-97): h + dt tend_h
     const double hin = S.h_in[i];
     const double hpi = S.fct ? rcp_nr(fma(S.dt, tend_h, hin)) : 0.0;
-    if (S.tape_hpi) S.tape_hpi[i] = hpi;
     if constexpr (SPLIT)
       S.hpw[i] = hpi;
     else
       cell_limiter<T, NC>(m, S, L, c, k, i, hin, hpi);
+    if (S.tape_hpi) S.tape_hpi[i] = hpi;
+  }
+  const double acc = fma(S.w_acc, tend_h, acc0);
+  if (S.stage == 3) {
+    S.h_new[i] = acc;
+  } else {
+    S.h_out[i] = fma(S.w_sub, tend_h, hp);
+    S.h_acc[i] = acc;
   }
 }
 
 template <int T, int NW, int OC, int SPLIT, int LANES = 1>
-__global__ void MPASO_BOUNDS(OC) k_sw_tend(DMesh m, DStat st, Stage S, int L) {
+__global__ void MPASO_BOUNDS(OC) k_sw_tend(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
   tend_item<T, NW, SPLIT, LANES>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
@@ -188,11 +185,12 @@ __global__ void MPASO_BOUNDS(OC) k_sw_tend(DMesh m, DStat st, Stage S, int L) {
 // Limiter kernel of the four-launch schedule: bounds, upwind tendency and
 // R+- of every cell from the fluxes k_sw_tend<.., SPLIT = 1> wrote.
 template <int T, int NC, int OC>
-__global__ void MPASO_BOUNDS(OC) k_sw_limit(DMesh m, Stage S, int L) {
+__global__ void MPASO_BOUNDS(OC) k_sw_limit(DMesh m, Stage S, Lev L) {
   stage_prologue();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   cell_limiter<T, NC>(m, S, L, c, k, i, S.h_in[i], S.hpw[i]);
 }
 
@@ -208,7 +206,8 @@ struct CellDiag {
   const DStat &st;
   const Stage &S;
   const double *u;
-  int L, k;
+  Lev L;
+  int k;
   double ke = 0.0, dv = 0.0;
   __device__ void operator()(int64_t s, int e, bool valid) {
     const double ue = u[(int64_t)e * L + k];
@@ -225,7 +224,7 @@ struct CellDiag {
 };
 
 template <int NC>
-__device__ __forceinline__ void cell_diag(const DMesh &m, const DStat &st, const Stage &S, int L,
+__device__ __forceinline__ void cell_diag(const DMesh &m, const DStat &st, const Stage &S, Lev L,
                                           int c, int k, int64_t i, const double *u) {
   CellDiag d{st, S, u, L, k};
   for_slots<NC>(m.nEoC[c], [&](int j, bool ok) {
@@ -235,7 +234,7 @@ __device__ __forceinline__ void cell_diag(const DMesh &m, const DStat &st, const
   d.finish(m, c, i);
 }
 
-__device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, const Stage &S, int L,
+__device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, const Stage &S, Lev L,
                                             int v, int k, int64_t i, const double *u,
                                             const double *h) {
   double circ = 0.0, hs = 0.0;
@@ -254,36 +253,37 @@ __device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, con
 
 // ------------------------------------------------------ K3: cells + vertices
 template <int T, int NC>
-__device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, const Stage &S, int L, int64_t i) {
+__device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
   const int64_t nCL = (int64_t)m.nC * L;
   const double *u_next = S.stage == 3 ? S.u_new : S.u_out;
   const double *h_next = S.stage == 3 ? S.h_new : S.h_out;
   if (i < nCL) {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     if constexpr (T > 0) {
-      const double hn = h_next[i];
+      const double hn = h_next[i], hpv = S.h_prev[i];
+      double tp[T], acc0[T];
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        tp[t] = S.tr_prev[i * T + t];
+        acc0[t] = S.stage == 0 ? 0.0 : S.trh_acc[i * T + t];
+      }
       // one pass over the cell's edges: tracer tendency and the next state's diagnostics
       CellDiag d{st, S, u_next, L, k};
       double tend[T];
       cell_tracer_tend<T, NC>(m, S, L, c, k, i, tend, d);
       d.finish(m, c, i);
       const double rh = rcp_nr(hn);
-      const double hpv = S.h_prev[i];
 #pragma unroll
       for (int t = 0; t < T; ++t) {
         // thickness-weighted tracer RK (apps/sw/tasks/solve.cc:162, 300-302, 337, 354)
-        const double hp_tp = hpv * S.tr_prev[i * T + t];
-        switch (S.stage) {
-          case 0:
-            S.tr_out[i * T + t] = fma(S.w_sub, tend[t], hp_tp) * rh;
-            S.trh_acc[i * T + t] = fma(S.w_acc, tend[t], hp_tp);
-            break;
-          case 3:
-            S.tr_new[i * T + t] = fma(S.w_acc, tend[t], S.trh_acc[i * T + t]) * rh;
-            break;
-          default:
-            S.tr_out[i * T + t] = fma(S.w_sub, tend[t], hp_tp) * rh;
-            S.trh_acc[i * T + t] = fma(S.w_acc, tend[t], S.trh_acc[i * T + t]);
+        const double hp_tp = hpv * tp[t];
+        const double acc = fma(S.w_acc, tend[t], S.stage == 0 ? hp_tp : acc0[t]);
+        if (S.stage == 3) {
+          S.tr_new[i * T + t] = acc * rh;
+        } else {
+          S.tr_out[i * T + t] = fma(S.w_sub, tend[t], hp_tp) * rh;
+          S.trh_acc[i * T + t] = acc;
         }
       }
     } else {
@@ -293,12 +293,13 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
   }
   i -= nCL;
   if (i >= (int64_t)m.nV * L) return;
-  const int v = (int)(i / L), k = (int)(i - (int64_t)v * L);
+  int v, k;
+  L.split(i, v, k);
   vertex_diag(m, st, S, L, v, k, i, u_next, h_next);
 }
 
 template <int T, int NC, int OC>
-__global__ void MPASO_BOUNDS(OC) k_sw_final(DMesh m, DStat st, Stage S, int L) {
+__global__ void MPASO_BOUNDS(OC) k_sw_final(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
   final_item<T, NC>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
@@ -306,17 +307,19 @@ __global__ void MPASO_BOUNDS(OC) k_sw_final(DMesh m, DStat st, Stage S, int L) {
 // Initial diagnostics (apps/sw/run.cc:88-92).
 // NC = 6: the cell loops unrolled for meshes of at most hexagons (as k_sw_final's unrolled variant)
 template <int NC>
-__global__ void __launch_bounds__(TPB) k_sw_diag(DMesh m, DStat st, Stage S, int L) {
+__global__ void __launch_bounds__(TPB) k_sw_diag(DMesh m, DStat st, Stage S, Lev L) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (i < nCL) {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     cell_diag<NC>(m, st, S, L, c, k, i, S.u_in);
     return;
   }
   i -= nCL;
   if (i >= (int64_t)m.nV * L) return;
-  const int v = (int)(i / L), k = (int)(i - (int64_t)v * L);
+  int v, k;
+  L.split(i, v, k);
   vertex_diag(m, st, S, L, v, k, i, S.u_in, S.h_in);
 }
 
@@ -364,7 +367,7 @@ __device__ bool grid_barrier(const GridBar &b, unsigned int &phase) {
 }
 
 template <int T, int NW, int NC>
-__global__ void __launch_bounds__(TPB) k_sw_persistent(DMesh m, DStat st, StageSet P, int L, int nsteps,
+__global__ void __launch_bounds__(TPB) k_sw_persistent(DMesh m, DStat st, StageSet P, Lev L, int nsteps,
                                                        GridBar b) {
   unsigned int phase = 0;
   const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nt = (int64_t)gridDim.x * blockDim.x;
@@ -524,7 +527,7 @@ Stage make_stage(SwState &s, int rk, double dt) {
 // (both travel into captured graphs with the launch).
 template <class... A>
 void launch_ex(void (*kern)(A...), int64_t n, int b, bool win, const SwState &s, cudaStream_t st,
-               DMesh m, DStat d, Stage S, int L) {
+               DMesh m, DStat d, Stage S, Lev L) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks_for(n, b));
   cfg.blockDim = dim3(b);
@@ -535,7 +538,7 @@ void launch_ex(void (*kern)(A...), int64_t n, int b, bool win, const SwState &s,
     at[na].id = cudaLaunchAttributeAccessPolicyWindow;
     at[na++].val.accessPolicyWindow = s.l2win;
   }
-  if (s.tune_pdl) {
+  if (stage_pdl(s)) {
     at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[na++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -592,9 +595,9 @@ void launch_k2(const SwState &s, const Stage &S, bool unroll, int b, cudaStream_
   if constexpr (SPLIT && T > 0) {
     const int64_t nc = (int64_t)m.nC * s.L;
     if (unroll)
-      launch_pdl(k_sw_limit<T, 6, OC>, nc, b, s.tune_pdl, st, m, S, s.L);
+      launch_pdl(k_sw_limit<T, 6, OC>, nc, b, stage_pdl(s), st, m, S, s.L);
     else
-      launch_pdl(k_sw_limit<T, 0, OC>, nc, b, s.tune_pdl, st, m, S, s.L);
+      launch_pdl(k_sw_limit<T, 0, OC>, nc, b, stage_pdl(s), st, m, S, s.L);
   }
 }
 
@@ -618,31 +621,31 @@ template <int T> void launch_stage_T(SwState &s, const Stage &S, cudaStream_t st
   const bool u1 = w10 && s.tune_unroll[0], u2 = w10 && c6 && s.tune_unroll[1];
   if (split) {  // K1 does the thickness flux part only (the T = 0 kernel)
     if (s.tune_occ[0])
-      launch_k1<0, 1>(s, S, u1, s.tune_tpb[0], st);
+      launch_k1<0, 1>(s, S, u1, stage_tpb(s, 0), st);
     else
-      launch_k1<0, 0>(s, S, u1, s.tune_tpb[0], st);
+      launch_k1<0, 0>(s, S, u1, stage_tpb(s, 0), st);
   } else if (OC1 && s.tune_occ[0]) {
-    launch_k1<T, OC1>(s, S, u1, s.tune_tpb[0], st);
+    launch_k1<T, OC1>(s, S, u1, stage_tpb(s, 0), st);
   } else {
-    launch_k1<T, 0>(s, S, u1, s.tune_tpb[0], st);
+    launch_k1<T, 0>(s, S, u1, stage_tpb(s, 0), st);
   }
   if (ev) prof_mark(ev[0], st);
   if (split) {
     if (OC1 && s.tune_occ[1])
-      launch_k2<T, OC1, 1>(s, S, u2, s.tune_tpb[1], st);
+      launch_k2<T, OC1, 1>(s, S, u2, stage_tpb(s, 1), st);
     else
-      launch_k2<T, 0, 1>(s, S, u2, s.tune_tpb[1], st);
+      launch_k2<T, 0, 1>(s, S, u2, stage_tpb(s, 1), st);
   } else if (OC1 && s.tune_occ[1]) {
-    launch_k2<T, OC1, 0>(s, S, u2, s.tune_tpb[1], st);
+    launch_k2<T, OC1, 0>(s, S, u2, stage_tpb(s, 1), st);
   } else {
-    launch_k2<T, 0, 0>(s, S, u2, s.tune_tpb[1], st);
+    launch_k2<T, 0, 0>(s, S, u2, stage_tpb(s, 1), st);
   }
   if (ev) prof_mark(ev[1], st);
   if (s.k2_mark) MPASO_CUDA(cudaEventRecord(s.k2_mark, st));
   if (OC1 && s.tune_occ[2])
-    launch_k3<T, OC1>(s, S, c6 && s.tune_unroll[2], s.tune_tpb[2], st);
+    launch_k3<T, OC1>(s, S, c6 && s.tune_unroll[2], stage_tpb(s, 2), st);
   else
-    launch_k3<T, 0>(s, S, c6 && s.tune_unroll[2], s.tune_tpb[2], st);
+    launch_k3<T, 0>(s, S, c6 && s.tune_unroll[2], stage_tpb(s, 2), st);
   if (ev) prof_mark(ev[2], st);
 }
 
@@ -692,7 +695,7 @@ void launch_persistent_T(SwState &s, const StageSet &P, int nsteps, GridBar b) {
   DMesh mm = m;
   DStat dd = s.st;
   StageSet pp = P;
-  int L = s.L;
+  Lev L = s.L;
   void *args[] = {&mm, &dd, &pp, &L, &nsteps, &b};
   MPASO_CUDA(cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(TPB), args, 0, s.stream));
 }
@@ -1541,6 +1544,7 @@ int mpaso_state_set_launch_config(mpaso_state s, const int32_t *config) {
       S.tune_unroll[k] = config[k], S.tune_tpb[k] = config[3 + k], S.tune_occ[k] = config[6 + k];
     set_l2_window(S, config[9]);
     S.tune_pdl = config[10];
+    S.tune_auto = false;
     S.tune_split = S.p.app == MPASO_APP_SW && S.T > 0 ? config[11] : 0;
   });
 }
@@ -1595,6 +1599,7 @@ int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *conf
     };
     try {
       drop_graph(S);
+      S.tune_auto = false;
       save_restore(true);
       double ms[3];
       time_stage_kernels(S, dt, 1, ms);  // warm-up

@@ -176,6 +176,9 @@ struct SwState {
   int tune_unroll[3] = {1, 1, 1};
   int tune_tpb[3] = {256, 256, 256};
   int tune_occ[3] = {0, 0, 0};
+  // until a configuration is set or tuned the launches go by the rules of
+  // stage_tpb() and stage_pdl()
+  bool tune_auto = true;
   // L2 residency of one static array across the step: 0 none, 1 the advection
   // coefficient pairs (read by K1), 2 the TRiSK weights (read by K2); the
   // window is attached to that kernel's launches (see set_l2_window)
@@ -198,6 +201,33 @@ struct SwState {
   size_t aux_bytes = 0;
   ~SwState();
 };
+
+// Threads per block of stage kernel k.  Untuned, sw app: 64.  A mesh that does
+// not fill the GPU spreads over four times the SMs 256-thread blocks would use,
+// and on one that does, the partial last wave and the edge / cell boundary
+// inside a block cost less (level-7 sphere, one FCT tracer: 375 us per step with
+// 64, 376 with 128, 395 with 256; level 6: 117 / 119 / 129; 64 x 64 plane: 60 /
+// 60 / 64).  Ocean app: 128 for the edges (level 6, 60 x 3: 628 / 627 / 651 us
+// per launch); the cell kernels 256 where their blocks fill every SM (cells 471 /
+// 467 / 455, final 384 / 382 / 363), else 128 (77 x 54 plane, 7 x 1: 96.7 / 94.5 /
+// 97.9 us per step).
+inline int stage_tpb(const SwState &s, int k) {
+  if (!s.tune_auto) return s.tune_tpb[k];
+  if (s.p.app != MPASO_APP_OCEAN) return 64;
+  const MeshCtx &c = s.mesh->ctx;
+  return k == 0 || (int64_t)c.d.nC * s.L < 1024LL * c.sms ? 128 : 256;
+}
+
+// Whether consecutive stage kernels of the sw app overlap their launches.
+// Untuned: where a kernel's threads leave most of every SM free (at most 256
+// edge-levels an SM), so that the next kernel's blocks can wait resident beside
+// them.  64 x 64 plane 60.2 -> 57.8 us per step, level 4 61.9 -> 57.9, level 5
+// 70.1 -> 66.0; above, the waiting blocks spread unevenly: 24,000 cells 86.7
+// -> 102.6, level 6 117 -> 138.
+inline bool stage_pdl(const SwState &s) {
+  const MeshCtx &c = s.mesh->ctx;
+  return s.tune_auto ? (int64_t)c.d.nE * s.L <= 256LL * c.sms : s.tune_pdl != 0;
+}
 
 // Allocates the state buffers listed as (pointer, doubles) in one arena.
 void alloc_arena(SwState &s, std::vector<std::pair<double **, int64_t>> &bufs);
@@ -230,14 +260,14 @@ void drop_adjoint_graph(SwState &s);
 // thickness as hx = s * h_e; dv, cp, cm, kd are the matching 1/s copies.
 // NA > 0: compile-time advection-stencil width (the mesh's maxAdv); 0 = runtime.
 template <int T, int NA, bool RO = true>
-__device__ __forceinline__ void edge_tracer_fluxes(const DMesh &m, const Stage &S, int L, int e, int k,
+__device__ __forceinline__ void edge_tracer_fluxes(const DMesh &m, const Stage &S, Lev L, int e, int k,
                                                    int64_t i, int64_t i1, int64_t i2, double F,
                                                    double hx, const double *dv, const double2 *cpm,
                                                    const double *kd) {
   double t1[T], t2[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) t1[t] = ld_in<RO>(&S.tr_in[i1 * T + t]), t2[t] = ld_in<RO>(&S.tr_in[i2 * T + t]);
-  const double dvF = __ldcs(&dv[e]) * F;
+  const double dvF = __ldcs(dv + (e)) * F;
   if (S.fct) {
     // low order: dv (max(0,F) tr1 + min(0,F) tr2) == dv F tr_upwind (ocean solve.cc:110-113)
     const bool up1 = dgt0(F);
@@ -249,14 +279,14 @@ __device__ __forceinline__ void edge_tracer_fluxes(const DMesh &m, const Stage &
     const int na = NA > 0 ? NA : m.maxAdv;
 #pragma unroll
     for (int a = 0; a < na; ++a) {
-      const int cell = __ldcs(&m.advCells[(int64_t)a * m.nE + e]);
-      const double2 c2 = __ldcs(&cpm[(int64_t)a * m.nE + e]);
+      const int cell = __ldcs(m.advCells + ((int64_t)a * m.nE + e));
+      const double2 c2 = __ldcs(cpm + ((int64_t)a * m.nE + e));
       const double cf = neg ? c2.y : c2.x;
       const double *tr = S.tr_in + ((int64_t)cell * L + k) * T;
 #pragma unroll
       for (int t = 0; t < T; ++t) s[t] = fma(cf, ld_in<RO>(&tr[t]), s[t]);
     }
-    const int mask = __ldcs(&m.hoMask[(int64_t)e * m.fctLev + k]);
+    const int mask = __ldcs(m.hoMask + ((int64_t)e * m.fctLev + k));
     // A = HO - LO, HO = F s; edges without the high-order mask take the centred
     // flux (solve.cc:222-225).  A branch, not a select: the mask is set almost
     // everywhere, and the centred flux would cost three more FP64 instructions
@@ -285,7 +315,7 @@ __device__ __forceinline__ void edge_tracer_fluxes(const DMesh &m, const Stage &
     for (int t = 0; t < T; ++t) S.LO[i * T + t] = 0.0;
   }
   if (S.hmix) {
-    const double hk = hx * __ldcs(&kd[e]);
+    const double hk = hx * __ldcs(kd + (e));
 #pragma unroll
     for (int t = 0; t < T; ++t) S.DF[i * T + t] = hk * (t2[t] - t1[t]);
   }
@@ -311,7 +341,7 @@ __device__ __forceinline__ double dmask(double v, bool valid) { return valid ? v
 
 // Cell bounds, upwind tendency and limiter factors R+ / R- (ocean solve.cc:194-267).
 template <int T, int NC>
-__device__ __forceinline__ void cell_limiter(const DMesh &m, const Stage &S, int L, int c, int k,
+__device__ __forceinline__ void cell_limiter(const DMesh &m, const Stage &S, Lev L, int c, int k,
                                              int64_t i, double hin, double hpi) {
   const int n = m.nEoC[c];
   double tl[T];
@@ -387,7 +417,7 @@ struct NoEdgeHook {
 // `hook(slot, edge, valid)` runs once per edge slot of the cell inside the
 // same loop (the sw driver folds the next state's cell diagnostics into it).
 template <int T, int NC, class Hook = NoEdgeHook>
-__device__ __forceinline__ void cell_tracer_tend(const DMesh &m, const Stage &S, int L, int c, int k,
+__device__ __forceinline__ void cell_tracer_tend(const DMesh &m, const Stage &S, Lev L, int c, int k,
                                                  int64_t i, double *tend, Hook &&hook = Hook()) {
   const int n = m.nEoC[c];
   double2 own[T];

@@ -17,20 +17,22 @@ constexpr int TPB = 256;
 // ---------------------------------------------------------------- sw tasks
 // apps/sw/tasks/solve.cc:31-39 (h_edge), :41-60 (circulation, vorticity),
 // :62-77 (ke), :81-92 (h_vertex, pv_vertex).
-__global__ void k_sw_diag_a(DMesh m, int L, const double *__restrict__ h, const double *__restrict__ u,
+__global__ void k_sw_diag_a(DMesh m, Lev L, const double *__restrict__ h, const double *__restrict__ u,
                             double *h_edge, double *h_vertex, double *circulation, double *vorticity,
                             double *ke, double *pv_vertex) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nEL = (int64_t)m.nE * L, nVL = (int64_t)m.nV * L, nCL = (int64_t)m.nC * L;
   if (i < nEL) {
-    const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+    int e, k;
+    L.split(i, e, k);
     const int2 c = m.coe[e];
     h_edge[i] = 0.5 * (h[(int64_t)c.x * L + k] + h[(int64_t)c.y * L + k]);
     return;
   }
   i -= nEL;
   if (i < nVL) {
-    const int v = (int)(i / L), k = (int)(i - (int64_t)v * L);
+    int v, k;
+    L.split(i, v, k);
     double circ = 0.0;
     for (int j = 0; j < kVertexDegree; ++j) {  // edges in ascending reference order
       const int e = m.eov[(int64_t)j * m.nV + v];
@@ -50,7 +52,8 @@ __global__ void k_sw_diag_a(DMesh m, int L, const double *__restrict__ h, const 
   }
   i -= nVL;
   if (i < nCL) {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     double s = 0.0;
     const int n = m.nEoC[c];
     for (int j = 0; j < n; ++j) {
@@ -63,24 +66,26 @@ __global__ void k_sw_diag_a(DMesh m, int L, const double *__restrict__ h, const 
 }
 
 // apps/sw/tasks/solve.cc:95-106: pv_edge(e) = 0 + 0.5 pv(v) over the edge's two vertices.
-__global__ void k_sw_diag_b(DMesh m, int L, const double *__restrict__ pv_vertex, double *pv_edge) {
+__global__ void k_sw_diag_b(DMesh m, Lev L, const double *__restrict__ pv_vertex, double *pv_edge) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   const int2 v = m.voe[e];
   const double a = 0.5 * pv_vertex[(int64_t)v.x * L + k], b = 0.5 * pv_vertex[(int64_t)v.y * L + k];
   pv_edge[i] = (0.0 + a) + b;  // two terms: order-free
 }
 
 // apps/sw/tasks/solve.cc:169-234
-__global__ void k_sw_tend(DMesh m, int L, double g, const double *__restrict__ h_edge,
+__global__ void k_sw_tend(DMesh m, Lev L, double g, const double *__restrict__ h_edge,
                           const double *__restrict__ h, const double *__restrict__ u,
                           const double *__restrict__ ke, const double *__restrict__ pv_edge,
                           double *tend_h, double *tend_u) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nEL = (int64_t)m.nE * L, nCL = (int64_t)m.nC * L;
   if (i < nEL) {
-    const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+    int e, k;
+    L.split(i, e, k);
     const int2 c = m.coe[e];
     const int n = m.nEoE[e];
     const double pve = pv_edge[i];
@@ -97,7 +102,8 @@ __global__ void k_sw_tend(DMesh m, int L, double g, const double *__restrict__ h
   }
   i -= nEL;
   if (i < nCL) {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     double t = 0;
     const int n = m.nEoC[c];
     for (int j = 0; j < n; ++j) {  // scatter order: ascending reference edge id
@@ -110,12 +116,13 @@ __global__ void k_sw_tend(DMesh m, int L, double g, const double *__restrict__ h
 }
 
 // apps/sw/tasks/solve.cc:237-270
-__global__ void k_sw_scalar_tend(DMesh m, int L, int T, const double *__restrict__ h_edge,
+__global__ void k_sw_scalar_tend(DMesh m, Lev L, int T, const double *__restrict__ h_edge,
                                  const double *__restrict__ u, const double *__restrict__ tr,
                                  double *tend) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const int n = m.nEoC[c];
   for (int t = 0; t < T; ++t) {
     double acc = 0.0;
@@ -170,12 +177,13 @@ __global__ void k_oc_ntf(int64_t n, const double *hE, const double *u, double *n
 }
 
 // apps/ocean/tasks/solve.cc:60-97
-__global__ void k_oc_provisional(DMesh m, int L, const double *__restrict__ h,
+__global__ void k_oc_provisional(DMesh m, Lev L, const double *__restrict__ h,
                                  const double *__restrict__ ntf, double *hProv, double *hProvInv,
                                  double *hNewInv, double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   if (k >= m.maxLevelCell[c]) return;
   const double dtInvAreaCell = dt / m.areaCell[c];
   double hp = h[i];
@@ -191,11 +199,12 @@ __global__ void k_oc_provisional(DMesh m, int L, const double *__restrict__ h,
 }
 
 // apps/ocean/tasks/solve.cc:99-118
-__global__ void k_oc_low_order(DMesh m, int L, int T, const double *__restrict__ ntf,
+__global__ void k_oc_low_order(DMesh m, Lev L, int T, const double *__restrict__ ntf,
                                const double *__restrict__ tr, double *lo) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   const int2 c = m.coe[e];
   const double f = ntf[i];
   const double ntf1 = (0.0 < f) ? f : 0.0;  // std::max(0.0, f)
@@ -206,11 +215,12 @@ __global__ void k_oc_low_order(DMesh m, int L, int T, const double *__restrict__
 }
 
 // apps/ocean/tasks/solve.cc:120-167 (coef3rdOrder = 0.25, :11)
-__global__ void k_oc_high_order(DMesh m, int L, int T, const double *__restrict__ ntf,
+__global__ void k_oc_high_order(DMesh m, Lev L, int T, const double *__restrict__ ntf,
                                 const double *__restrict__ tr, double *ho) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   const double f = ntf[i];
   const double wgt = f * (double)m.hoMask[(int64_t)e * m.fctLev + k];
   const double sgn = (f < 0.0) ? -1.0 : (f > 0. ? 1.0 : 0.0);
@@ -230,13 +240,14 @@ __global__ void k_oc_high_order(DMesh m, int L, int T, const double *__restrict_
 }
 
 // apps/ocean/tasks/solve.cc:194-229: bounds (cells) and anti-diffusive flux (edges).
-__global__ void k_oc_fct_a(DMesh m, int L, int T, const double *__restrict__ ntf,
+__global__ void k_oc_fct_a(DMesh m, Lev L, int T, const double *__restrict__ ntf,
                            const double *__restrict__ lo, const double *__restrict__ tr, double *ho,
                            double *flxIn, double *flxOut, double *trMax, double *trMin) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L, nEL = (int64_t)m.nE * L;
   if (i < nCL) {
-    const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+    int c, k;
+    L.split(i, c, k);
     const int mlc = m.maxLevelCell[c];
     if (k < mlc) {
       const int n = m.nEoC[c];
@@ -260,7 +271,8 @@ __global__ void k_oc_fct_a(DMesh m, int L, int T, const double *__restrict__ ntf
   }
   i -= nCL;
   if (i < nEL) {
-    const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+    int e, k;
+    L.split(i, e, k);
     if (k >= m.maxLevelEdgeTop[e]) return;
     const int2 c = m.coe[e];
     const double tw = (double)((m.hoMask[(int64_t)e * m.fctLev + k] + 1) & 1) * (m.dvEdge[e] * 0.5) * ntf[i];
@@ -274,7 +286,7 @@ __global__ void k_oc_fct_a(DMesh m, int L, int T, const double *__restrict__ ntf
 }
 
 // apps/ocean/tasks/solve.cc:232-267: per-cell sums and limiter factors.
-__global__ void k_oc_fct_b(DMesh m, int L, int T, const double *__restrict__ hProvInv,
+__global__ void k_oc_fct_b(DMesh m, Lev L, int T, const double *__restrict__ hProvInv,
                            const double *__restrict__ h, const double *__restrict__ lo,
                            const double *__restrict__ tr, const double *__restrict__ ho,
                            double *flxIn, double *flxOut, double *tend,
@@ -282,7 +294,8 @@ __global__ void k_oc_fct_b(DMesh m, int L, int T, const double *__restrict__ hPr
                            double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const double eps = 1.e-10;
   const double invAreaCell1 = 1.0 / m.areaCell[c];
   const int n = m.nEoC[c];
@@ -318,11 +331,12 @@ __global__ void k_oc_fct_b(DMesh m, int L, int T, const double *__restrict__ hPr
 }
 
 // apps/ocean/tasks/solve.cc:270-282: rescale anti-diffusive fluxes.
-__global__ void k_oc_fct_c(DMesh m, int L, int T, const double *__restrict__ flxIn,
+__global__ void k_oc_fct_c(DMesh m, Lev L, int T, const double *__restrict__ flxIn,
                            const double *__restrict__ flxOut, double *ho) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  const int e = (int)(i / L), k = (int)(i - (int64_t)e * L);
+  int e, k;
+  L.split(i, e, k);
   if (k >= m.maxLevelEdgeTop[e]) return;
   const int2 c = m.coe[e];
   for (int t = 0; t < T; ++t) {
@@ -335,13 +349,14 @@ __global__ void k_oc_fct_c(DMesh m, int L, int T, const double *__restrict__ flx
 }
 
 // apps/ocean/tasks/solve.cc:287-326
-__global__ void k_oc_accumulate_fct(DMesh m, int L, int T, const double *__restrict__ hProvInv,
+__global__ void k_oc_accumulate_fct(DMesh m, Lev L, int T, const double *__restrict__ hProvInv,
                                     const double *__restrict__ h, const double *__restrict__ ho,
                                     const double *__restrict__ tr, double *trProv, double *tend,
                                     double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const double invAreaCell1 = 1.0 / m.areaCell[c];
   const int n = m.nEoC[c];
   for (int t = 0; t < T; ++t) {
@@ -357,11 +372,12 @@ __global__ void k_oc_accumulate_fct(DMesh m, int L, int T, const double *__restr
 }
 
 // apps/ocean/tasks/solve.cc:328-366
-__global__ void k_oc_hmix(DMesh m, int L, int T, const double *__restrict__ hE,
+__global__ void k_oc_hmix(DMesh m, Lev L, int T, const double *__restrict__ hE,
                           const double *__restrict__ tr, double *tend, double coef) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
-  const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
+  int c, k;
+  L.split(i, c, k);
   const double invArea = 1.0 / m.areaCell[c];
   const int n = m.nEoC[c];
   for (int t = 0; t < T; ++t) {
