@@ -115,6 +115,14 @@ struct MeshCtx {
   int32_t *d_iperm[3] = {nullptr, nullptr, nullptr};  // device copies of iperm
   void *arena = nullptr;
   size_t arena_bytes = 0;
+  // The arrays the per-task kernels read, in the reference's numbering, so that
+  // those kernels run on the caller's fields where they lie (built by the first
+  // task call; `d` itself where the context keeps the reference's numbering).
+  DMesh ref{};
+  bool has_ref = false;
+  void *ref_arena = nullptr;
+  size_t ref_bytes = 0;
+  const DMesh &task_view();
   // growable scratch for the per-task entries
   void *scratch = nullptr;
   size_t scratch_bytes = 0;

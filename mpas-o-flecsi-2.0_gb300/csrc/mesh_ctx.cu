@@ -14,6 +14,7 @@ namespace mpaso {
 MeshCtx::~MeshCtx() {
   if (arena) cudaFree(arena);
   if (scratch) cudaFree(scratch);
+  if (ref_arena) cudaFree(ref_arena);
   if (geo) cudaFree(geo);
   for (auto &p : d_perm)
     if (p) cudaFree(p);
@@ -740,8 +741,8 @@ int mpaso_mesh_device_bytes(mpaso_mesh m, int64_t *bytes) {
   return mpaso::guarded("mpaso_mesh_device_bytes", [&] {
     mpaso::require(m && bytes, MPASO_ERR_ARG, "null argument");
     const mpaso::DMesh &d = m->ctx.d;
-    // the arena, the per-task scratch and both permutations of each entity
-    *bytes = (int64_t)(m->ctx.arena_bytes + m->ctx.scratch_bytes) + 2 * 4 * (d.nC + d.nE + d.nV);
+    // the arena, the per-task scratch and view, and both permutations of each entity
+    *bytes = (int64_t)(m->ctx.arena_bytes + m->ctx.scratch_bytes + m->ctx.ref_bytes) + 2 * 4 * (d.nC + d.nE + d.nV);
   });
 }
 

@@ -1,6 +1,6 @@
-// Staging of per-task arguments: reference-numbered host or device arrays are
-// gathered into the context's Hilbert numbering before a task kernel runs and
-// scattered back afterwards.
+// Arguments of the per-task entries.  The task kernels run in the reference's
+// numbering (MeshCtx::task_view) on device arrays where they lie; host arrays
+// are copied in and back out.
 #pragma once
 
 #include "device.cuh"
@@ -28,30 +28,31 @@ class TaskIO {
   TaskIO(mpaso_mesh m, void *stream);
   ~TaskIO();
   // Registers an argument; returns its slot.  `entity` = MPASO_CELLS/EDGES/VERTICES,
-  // `row` = doubles per entity.  Outputs are copied in as well, so entries a task
-  // leaves untouched keep their values (FleCSI storage semantics).
+  // `row` = doubles per entity.  Entries of an output that a task leaves untouched
+  // keep their values (FleCSI storage semantics): staged outputs are copied in as well.
   int in(const double *p, int entity, int row) { return add(p, entity, row, false); }
   int out(double *p, int entity, int row) { return add(p, entity, row, true); }
-  void stage();                  // copies + gathers into the internal layout
+  void stage();                  // copies host arrays in
   double *ptr(int slot) const { return args_[slot].internal; }
-  void finish();                 // scatters outputs back, syncs for host memory
+  void finish();                 // copies outputs back, syncs for host memory
   cudaStream_t stream() const { return stream_; }
   MeshCtx &ctx() { return m_->ctx; }
-  const DMesh &dm() const { return m_->ctx.d; }
+  const DMesh &dm() const { return m_->ctx.ref; }  // reference numbering, valid after stage()
 
  private:
   struct Arg {
     double *user;
     int entity, row;
     bool output, host;
-    double *internal = nullptr, *raw = nullptr;
+    double *internal = nullptr;
   };
   int add(const double *p, int entity, int row, bool output);
   int64_t count(int entity) const;
+  bool overlapping() const;
   mpaso_mesh m_;
   cudaStream_t stream_;
   std::vector<Arg> args_;
-  bool any_host_ = false;
+  bool any_host_ = false, copies_ = false;
 };
 
 }  // namespace mpaso
