@@ -142,6 +142,7 @@ inline int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) /
 // --------------------------------------------------- FP64 helpers (INT pipe)
 // GB300 issues FP64 at a small fraction of its integer rate, so selects,
 // min/max, sign tests and sign flips on doubles are done on bit patterns.
+constexpr long long kSignBit = (long long)0x8000000000000000ULL;
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 __device__ __forceinline__ double bitsd(long long b) { return __longlong_as_double(b); }
 

@@ -79,14 +79,6 @@ __global__ void k_oc_prep(DMesh m, int L, const double *u, const double *h, cons
   hpi[i] = 1.0 / hp;
 }
 
-// Rare work of K1, called so that warps without it skip it: inlined, it becomes
-// predicated instructions, which occupy the FP64 pipe all the same (11 a
-// thread beside the 36 sums of three tracers).
-__device__ __noinline__ double masked_weight(double f, int mask) { return f * (double)mask; }
-__device__ __noinline__ double add_centred_flux(double flx, double dv, double f, double t1, double t2) {
-  return flx + (dv * 0.5) * f * (t1 + t2);
-}
-
 // K1: per edge-level, for every tracer, the low-order flux LO
 // (solve.cc:106-116), the high-order flux corrected for FCT, A = HO - LO
 // (solve.cc:143-165, 216-229), and the del2 flux DF = hE (tr2 - tr1) rho
@@ -174,15 +166,6 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
       S.DF[i * T + t] = x;
     }
   }
-}
-
-// min(1, max(0, num / den)) for den > 0, divided only strictly inside (0, 1):
-// num <= 0 gives 0 and num >= den gives 1 exactly as the clamped quotient does.
-__device__ __forceinline__ double clamp_quotient(double num, double den) {
-  if (!dgt0(den)) return dclamp01(num / den);
-  if (!dgt0(num)) return 0.0;
-  if (!(dkey(num) < dkey(den))) return 1.0;
-  return dclamp01(num / den);
 }
 
 // K2: per cell-level, for every tracer, the bounds over the cell and its

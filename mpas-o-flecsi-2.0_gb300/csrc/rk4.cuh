@@ -9,8 +9,6 @@
 
 namespace mpaso {
 
-constexpr long long kSignBit = (long long)0x8000000000000000ULL;
-
 // Fast FP64 reciprocal: hardware approximation (rcp.approx.ftz.f64) refined
 // by two Newton-Raphson steps r <- r + r (1 - b r); within a few ulp of 1/b
 // for normal b.

@@ -94,4 +94,23 @@ __device__ __forceinline__ double mul_int(double a, double b) {
   return r;
 }
 
+// Rare work of the high-order flux, called so that warps without it skip it: inlined, it becomes
+// predicated instructions, which occupy the FP64 pipe all the same (11 a
+// thread beside the 36 sums of three tracers).
+static __device__ __noinline__ double masked_weight(double f, int mask) { return f * (double)mask; }
+static __device__ __noinline__ double add_centred_flux(double flx, double dv, double f, double t1, double t2) {
+  return flx + (dv * 0.5) * f * (t1 + t2);
+}
+
+// num / den where few lanes need it (a call, as product_outside).
+static __device__ __noinline__ double rare_quotient(double num, double den) { return num / den; }
+
+// min(1, max(0, num / den)) for den > 0, divided only strictly inside (0, 1):
+// num <= 0 gives 0 and num >= den gives 1 exactly as the clamped quotient does.
+__device__ __forceinline__ double clamp_quotient(double num, double den) {
+  double r = dgt0(num) ? 1.0 : 0.0;
+  if (!dgt0(den) || (dgt0(num) && dkey(num) < dkey(den))) r = dclamp01(rare_quotient(num, den));
+  return r;
+}
+
 }  // namespace mpaso

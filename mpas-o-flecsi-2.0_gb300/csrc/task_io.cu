@@ -107,7 +107,7 @@ int64_t TaskIO::count(int entity) const {
 int TaskIO::add(const double *p, int entity, int row, bool output) {
   require(p != nullptr, MPASO_ERR_ARG, "null field pointer");
   require(row >= 1, MPASO_ERR_ARG, "bad row length");
-  Arg a{const_cast<double *>(p), entity, row, output, !is_device_pointer(p)};
+  Arg a{const_cast<double *>(p), entity, row, output, !is_device_pointer(p), false};
   any_host_ |= a.host;
   args_.push_back(a);
   return (int)args_.size() - 1;
@@ -121,7 +121,7 @@ bool TaskIO::overlapping() const {
     const double *x0 = args_[x].user, *x1 = x0 + count(args_[x].entity) * args_[x].row;
     for (size_t y = 0; y < args_.size(); ++y) {
       const double *y0 = args_[y].user, *y1 = y0 + count(args_[y].entity) * args_[y].row;
-      if (x != y && x0 < y1 && y0 < x1) return true;
+      if (x != y && !args_[y].work && x0 < y1 && y0 < x1) return true;
     }
   }
   return false;
@@ -133,15 +133,16 @@ void TaskIO::stage() {
   size_t total = 0;
   auto bytes_of = [&](const Arg &a) { return (size_t)count(a.entity) * a.row * sizeof(double); };
   for (auto &a : args_)
-    if (a.host || copies_) total += (bytes_of(a) + 255) & ~size_t(255);
+    if (a.host || a.work || copies_) total += (bytes_of(a) + 255) & ~size_t(255);
   char *base = total ? (char *)m_->ctx.ensure_scratch(total) : nullptr;
   for (auto &a : args_) {
-    if (!a.host && !copies_) {
+    if (!a.host && !a.work && !copies_) {
       a.internal = a.user;
       continue;
     }
     a.internal = (double *)base;
     base += (bytes_of(a) + 255) & ~size_t(255);
+    if (a.work) continue;
     MPASO_CUDA(cudaMemcpyAsync(a.internal, a.user, bytes_of(a),
                                a.host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, stream_));
   }
@@ -213,7 +214,7 @@ const DMesh &MeshCtx::task_view() {
       {&m.nEoE, 4, MPASO_EDGES, 1, -1, false}, {&m.eoe, 4, MPASO_EDGES, E, MPASO_EDGES, false},
       {&m.woe, 8, MPASO_EDGES, E, -1, false}, {&m.maxLevelEdgeTop, 4, MPASO_EDGES, 1, -1, false},
       {&m.nAdv, 4, MPASO_EDGES, 1, -1, false}, {&m.advCells, 4, MPASO_EDGES, d.maxAdv, MPASO_CELLS, false},
-      {&m.advCoef, 8, MPASO_EDGES, d.maxAdv, -1, false}, {&m.advCoef3, 8, MPASO_EDGES, d.maxAdv, -1, false},
+      {&m.advCp, 8, MPASO_EDGES, d.maxAdv, -1, false}, {&m.advCm, 8, MPASO_EDGES, d.maxAdv, -1, false},
       {&m.hoMask, 4, MPASO_EDGES, d.fctLev, -1, true}, {&m.meshScalingDel2, 8, MPASO_EDGES, 1, -1, false},
       {&m.cov, 4, MPASO_VERTICES, kVertexDegree, MPASO_CELLS, false},
       {&m.kite, 8, MPASO_VERTICES, kVertexDegree, -1, false},
@@ -254,7 +255,7 @@ const DMesh &MeshCtx::task_view() {
     throw;
   }
   // what no task kernel reads keeps no pointer into the other numbering
-  m.nbr = nullptr, m.invDcEdge = m.invDvEdge = nullptr, m.advCp = m.advCm = nullptr, m.invAreaTriangle = nullptr;
+  m.nbr = nullptr, m.invDcEdge = m.invDvEdge = nullptr, m.advCoef = m.advCoef3 = nullptr, m.invAreaTriangle = nullptr;
   m.woeT = m.kiteR = nullptr, m.vocR = m.advRe = m.cocU = nullptr, m.advRc = nullptr;
   ref = m, ref_arena = arena_new, ref_bytes = total, has_ref = true;
   return ref;

@@ -1,12 +1,16 @@
 // Per-task kernels: one GPU kernel set per reference task, same signature and
-// semantics, operating on the context's renumbered HBM layout.
+// semantics, operating on the caller's fields in the reference's numbering.
 //
 // Each kernel evaluates every output element with the same sequence of IEEE
 // operations as the reference loop it cites (this file is compiled with
 // -fmad=false, so no multiply-add is fused), and scatter loops of the
 // reference become gathers over the reverse connectivity in the order the
-// scatter visited them.  Results therefore agree bit for bit with the
-// reference tasks.  One thread per (entity, level); tracers loop inside.
+// scatter visited them.  Results therefore agree value for value with the
+// reference tasks (bit for bit, signs of zero in the ocean tasks aside).  One
+// thread per (entity, level); tracers loop inside.
+#include <type_traits>
+
+#include "softmul.cuh"
 #include "task_io.cuh"
 
 namespace mpaso {
@@ -176,10 +180,38 @@ __global__ void k_oc_ntf(int64_t n, const double *hE, const double *u, double *n
   if (i < n) ntf[i] = u[i] * hE[i];  // apps/ocean/tasks/solve.cc:49-54
 }
 
+// The products of the kernels below run on the integer pipe (softmul.cuh, the
+// hardware's rounding bit for bit) and comparisons on the bit patterns, which
+// leaves the FP64 pipe the sums; tracers are unrolled at compile time, and what
+// levels share (1 / area, the mixing coefficient) is not divided out in each.
+// Level 5, 20 levels x 3 tracers, us: high order 130 -> 63, fct_a + fct_b + fct_c
+// 187 -> 83, hmix 128 -> 36, accumulate 35 -> 20, low order 20 -> 11, provisional
+// 20 -> 16; a tracer stage task by task 456 -> 184.
+
+// IEEE a < b on the integer pipe (false with a NaN; zeros are equal).
+__device__ __forceinline__ bool ieee_lt(double a, double b) {
+  constexpr long long kInf = 0x7ff0000000000000LL;
+  const long long x = dbits(a), y = dbits(b);
+  const long long ka = x < 0 ? kSignBit - x : x, kb = y < 0 ? kSignBit - y : y;
+  return ka < kb && kb <= kInf && ka >= -kInf;
+}
+
+static __device__ __noinline__ double rare_product(double a, double b) { return a * b; }
+
+// s * x for an edge sign s: a sign flip for the +-1 it is, else the product.
+struct EdgeSign {
+  double s;
+  long long flip;
+  bool unit;
+  __device__ explicit EdgeSign(double v)
+      : s(v), flip(dbits(v) & kSignBit), unit((dbits(v) & ~kSignBit) == 0x3ff0000000000000LL) {}
+  __device__ double times(double x) const { return unit ? dflip(x, flip) : rare_product(s, x); }
+};
+
 // apps/ocean/tasks/solve.cc:60-97
-__global__ void k_oc_provisional(DMesh m, Lev L, const double *__restrict__ h,
-                                 const double *__restrict__ ntf, double *hProv, double *hProvInv,
-                                 double *hNewInv, double dt) {
+__global__ void __launch_bounds__(TPB) k_oc_provisional(DMesh m, Lev L, const double *__restrict__ h,
+                                                        const double *__restrict__ ntf, double *hProv,
+                                                        double *hProvInv, double *hNewInv, double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
   int c, k;
@@ -189,211 +221,305 @@ __global__ void k_oc_provisional(DMesh m, Lev L, const double *__restrict__ h,
   double hp = h[i];
   const int n = m.nEoC[c];
   for (int j = 0; j < n; ++j) {
-    const int e = m.eoc[(int64_t)j * m.nC + c];
-    const double sf = dtInvAreaCell * m.dvEdge[e] * m.eocSign[(int64_t)j * m.nC + c];
-    hp += sf * ntf[(int64_t)e * L + k];
+    const int64_t s = (int64_t)j * m.nC + c;
+    const int e = m.eoc[s];
+    const double sf = EdgeSign(m.eocSign[s]).times(mul_int(m.dvEdge[e], dtInvAreaCell));
+    hp += mul_int(ntf[(int64_t)e * L + k], sf);
   }
   hProv[i] = hp;
-  hProvInv[i] = 1.0 / hp;
-  hNewInv[i] = 1.0 / hp;
+  const double inv = 1.0 / hp;
+  hProvInv[i] = inv;
+  hNewInv[i] = inv;
 }
 
-// apps/ocean/tasks/solve.cc:99-118
-__global__ void k_oc_low_order(DMesh m, Lev L, int T, const double *__restrict__ ntf,
-                               const double *__restrict__ tr, double *lo) {
+// max(0, f) tr1 + min(0, f) tr2 where a factor is not finite or outside the products' window
+static __device__ __noinline__ double rare_upwind(double f, double tr1, double tr2) {
+  const double ntf1 = (0.0 < f) ? f : 0.0;  // std::max(0.0, f)
+  const double ntf2 = (f < 0.0) ? f : 0.0;  // std::min(0.0, f)
+  return ntf1 * tr1 + ntf2 * tr2;
+}
+
+// apps/ocean/tasks/solve.cc:99-118: dv (max(0, f) tr1 + min(0, f) tr2), one of
+// whose two products is a zero
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_low_order(DMesh m, Lev L, const double *__restrict__ ntf,
+                                                      const double *__restrict__ tr, double *lo) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
   int e, k;
   L.split(i, e, k);
   const int2 c = m.coe[e];
-  const double f = ntf[i];
-  const double ntf1 = (0.0 < f) ? f : 0.0;  // std::max(0.0, f)
-  const double ntf2 = (f < 0.0) ? f : 0.0;  // std::min(0.0, f)
-  for (int t = 0; t < T; ++t)
-    lo[i * T + t] = m.dvEdge[e] * (ntf1 * tr[((int64_t)c.x * L + k) * T + t] +
-                                   ntf2 * tr[((int64_t)c.y * L + k) * T + t]);
+  const double f = ntf[i], dv = m.dvEdge[e];
+  const int64_t i1 = ((int64_t)c.x * L + k) * T, i2 = ((int64_t)c.y * L + k) * T;
+  uint32_t badf = 0, badv = 0;
+  const SoftFactor ff = soft_factor(f, badf), fv = soft_factor(dv, badv);
+  constexpr long long kInf = 0x7ff0000000000000LL;
+  const bool up1 = dgt0(f);
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const double t1 = tr[i1 + t], t2 = tr[i2 + t];
+    uint32_t bad = badf;
+    double x = soft_mul(up1 ? t1 : t2, ff, bad);
+    if (bad || (dbits(up1 ? t2 : t1) & kInf) == kInf) x = rare_upwind(f, t1, t2);
+    bad = badv;
+    double r = soft_mul(x, fv, bad);
+    if (bad) r = rare_product(dv, x);
+    lo[i * T + t] = r;
+  }
 }
 
-// apps/ocean/tasks/solve.cc:120-167 (coef3rdOrder = 0.25, :11)
-__global__ void k_oc_high_order(DMesh m, Lev L, int T, const double *__restrict__ ntf,
-                                const double *__restrict__ tr, double *ho) {
+// apps/ocean/tasks/solve.cc:120-167 (coef3rdOrder = 0.25, :11).  The factor
+// coef1 + coef3 sgn is advCp / advCm by the sign of the flux (a zero flux
+// weighs every term with zero).
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_high_order(DMesh m, Lev L, const double *__restrict__ ntf,
+                                                       const double *__restrict__ tr, double *ho) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
   int e, k;
   L.split(i, e, k);
   const double f = ntf[i];
-  const double wgt = f * (double)m.hoMask[(int64_t)e * m.fctLev + k];
-  const double sgn = (f < 0.0) ? -1.0 : (f > 0. ? 1.0 : 0.0);
-  double flx[kMaxTracers];
+  const int mask = m.hoMask[(int64_t)e * m.fctLev + k];
+  const double wgt = mask == 1 ? f : mask == 0 ? bitsd(dbits(f) & kSignBit) : masked_weight(f, mask);
+  const double *coef = dlt0(f) ? m.advCm : m.advCp;
+  uint32_t badw = 0;
+  const SoftFactor fw = soft_factor(wgt, badw);
+  double flx[T];
+#pragma unroll
   for (int t = 0; t < T; ++t) flx[t] = 0.0;
   const int n = m.nAdv[e];
+#pragma unroll 2
   for (int a = 0; a < n; ++a) {
-    const int cell = m.advCells[(int64_t)a * m.nE + e];
-    const double coef1 = m.advCoef[(int64_t)a * m.nE + e];
-    const double coef3 = m.advCoef3[(int64_t)a * m.nE + e] * 0.25;
-    if (k < m.maxLevelCell[cell]) {
-      const double wf = wgt * (coef1 + coef3 * sgn);
-      for (int t = 0; t < T; ++t) flx[t] += tr[((int64_t)cell * L + k) * T + t] * wf;
+    const int64_t sa = (int64_t)a * m.nE + e;
+    const int cell = m.advCells[sa];
+    if (k >= m.maxLevelCell[cell]) continue;
+    const double cf = coef[sa];
+    const double *x = tr + ((int64_t)cell * L + k) * T;
+    uint32_t bad = badw;
+    const SoftFactor wf = soft_factor(soft_mul(cf, fw, bad), bad);
+    double p[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) p[t] = soft_mul(x[t], wf, bad);
+    if (bad) {
+      const double wx = rare_product(wgt, cf);
+#pragma unroll
+      for (int t = 0; t < T; ++t) p[t] = rare_product(x[t], wx);
     }
+#pragma unroll
+    for (int t = 0; t < T; ++t) flx[t] += p[t];
   }
+#pragma unroll
   for (int t = 0; t < T; ++t) ho[i * T + t] = flx[t];
 }
 
-// apps/ocean/tasks/solve.cc:194-229: bounds (cells) and anti-diffusive flux (edges).
-__global__ void k_oc_fct_a(DMesh m, Lev L, int T, const double *__restrict__ ntf,
-                           const double *__restrict__ lo, const double *__restrict__ tr, double *ho,
-                           double *flxIn, double *flxOut, double *trMax, double *trMin) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t nCL = (int64_t)m.nC * L, nEL = (int64_t)m.nE * L;
-  if (i < nCL) {
-    int c, k;
-    L.split(i, c, k);
-    const int mlc = m.maxLevelCell[c];
-    if (k < mlc) {
-      const int n = m.nEoC[c];
-      for (int t = 0; t < T; ++t) {
-        double mx = tr[i * T + t], mn = mx;
-        for (int j = 0; j < n; ++j) {
-          const int c2 = m.coc[(int64_t)j * m.nC + c];
-          if (k < min(mlc, m.maxLevelCell[c2])) {
-            const double x = tr[((int64_t)c2 * L + k) * T + t];
-            mx = (mx < x) ? x : mx;  // std::max
-            mn = (x < mn) ? x : mn;  // std::min
-          }
-        }
-        trMax[i * T + t] = mx;
-        trMin[i * T + t] = mn;
-        flxIn[i * T + t] = 0.0;
-        flxOut[i * T + t] = 0.0;
-      }
-    }
-    return;
-  }
-  i -= nCL;
-  if (i < nEL) {
-    int e, k;
-    L.split(i, e, k);
-    if (k >= m.maxLevelEdgeTop[e]) return;
+// apps/ocean/tasks/solve.cc:216-229: anti-diffusive flux of the edges.  The
+// centred flux has the weight ((mask + 1) & 1), which is 0 on almost all of them.
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_fct_a(DMesh m, Lev L, const double *__restrict__ ntf,
+                                                  const double *__restrict__ lo, const double *__restrict__ tr,
+                                                  double *ho) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= (int64_t)m.nE * L) return;
+  int e, k;
+  L.split(i, e, k);
+  if (k >= m.maxLevelEdgeTop[e]) return;
+  const bool centred = (m.hoMask[(int64_t)e * m.fctLev + k] + 1) & 1;
+  double x[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) x[t] = ho[i * T + t];
+  if (centred) {
     const int2 c = m.coe[e];
-    const double tw = (double)((m.hoMask[(int64_t)e * m.fctLev + k] + 1) & 1) * (m.dvEdge[e] * 0.5) * ntf[i];
-    for (int t = 0; t < T; ++t) {
-      double x = ho[i * T + t];
-      x += tw * (tr[((int64_t)c.x * L + k) * T + t] + tr[((int64_t)c.y * L + k) * T + t]);
-      x -= lo[i * T + t];
-      ho[i * T + t] = x;
-    }
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+      x[t] = add_centred_flux(x[t], m.dvEdge[e], ntf[i], tr[((int64_t)c.x * L + k) * T + t],
+                              tr[((int64_t)c.y * L + k) * T + t]);
   }
+#pragma unroll
+  for (int t = 0; t < T; ++t) ho[i * T + t] = x[t] - lo[i * T + t];
 }
 
-// apps/ocean/tasks/solve.cc:232-267: per-cell sums and limiter factors.
-__global__ void k_oc_fct_b(DMesh m, Lev L, int T, const double *__restrict__ hProvInv,
-                           const double *__restrict__ h, const double *__restrict__ lo,
-                           const double *__restrict__ tr, const double *__restrict__ ho,
-                           double *flxIn, double *flxOut, double *tend,
-                           const double *__restrict__ trMax, const double *__restrict__ trMin,
-                           double dt) {
+// apps/ocean/tasks/solve.cc:194-214, 232-267: bounds over the cell and its
+// neighbours, per-cell sums and limiter factors.
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_fct_b(DMesh m, Lev L, const double *__restrict__ hProvInv,
+                                                  const double *__restrict__ h, const double *__restrict__ lo,
+                                                  const double *__restrict__ tr, const double *__restrict__ ho,
+                                                  double *flxIn, double *flxOut, double *tend, double *trMax,
+                                                  double *trMin, double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
   int c, k;
   L.split(i, c, k);
   const double eps = 1.e-10;
-  const double invAreaCell1 = 1.0 / m.areaCell[c];
-  const int n = m.nEoC[c];
+  const double invAreaCell1 = m.invAreaCell[c];  // 1 / areaCell
+  const int n = m.nEoC[c], mlc = m.maxLevelCell[c];
+  const bool live = k < mlc;
+  double trc[T], mx[T], mn[T], td[T], fin[T], fout[T];
+#pragma unroll
   for (int t = 0; t < T; ++t) {
-    double td = tend[i * T + t], fin = flxIn[i * T + t], fout = flxOut[i * T + t];
-    for (int j = 0; j < n; ++j) {
-      const int e = m.eoc[(int64_t)j * m.nC + c];
-      if (k < m.maxLevelEdgeTop[e]) {
-        const double sf = m.eocSign[(int64_t)j * m.nC + c] * invAreaCell1;
-        td += sf * lo[((int64_t)e * L + k) * T + t];
-        const double x = sf * ho[((int64_t)e * L + k) * T + t];
-        fin += (0.0 < x) ? x : 0.0;
-        fout += (x < 0.0) ? x : 0.0;
+    const int64_t it = i * T + t;
+    trc[t] = mx[t] = mn[t] = tr[it];
+    td[t] = tend[it];
+    fin[t] = live ? 0.0 : flxIn[it], fout[t] = live ? 0.0 : flxOut[it];
+  }
+  for (int j = 0; j < n; ++j) {
+    const int64_t s = (int64_t)j * m.nC + c;
+    const int e = m.eoc[s], c2 = m.coc[s];
+    if (live && k < m.maxLevelCell[c2]) {
+#pragma unroll
+      for (int t = 0; t < T; ++t) {
+        const double x = tr[((int64_t)c2 * L + k) * T + t];
+        mx[t] = ieee_lt(mx[t], x) ? x : mx[t];  // std::max
+        mn[t] = ieee_lt(x, mn[t]) ? x : mn[t];  // std::min
       }
     }
-    tend[i * T + t] = td;
-    if (k < m.maxLevelCell[c]) {
-      const double hpi = hProvInv[i];
-      const double up = (tr[i * T + t] * h[i] + dt * td) * hpi;
-      const double mxn = up + dt * fin * hpi;
-      const double mnn = up + dt * fout * hpi;
-      double sfac = (trMax[i * T + t] - up) / (mxn - up + eps);
-      sfac = (0.0 < sfac) ? sfac : 0.0;
-      flxIn[i * T + t] = (sfac < 1.0) ? sfac : 1.0;
-      sfac = (up - trMin[i * T + t]) / (up - mnn + eps);
-      sfac = (0.0 < sfac) ? sfac : 0.0;
-      flxOut[i * T + t] = (sfac < 1.0) ? sfac : 1.0;
-    } else {
-      flxIn[i * T + t] = fin;
-      flxOut[i * T + t] = fout;
+    if (k >= m.maxLevelEdgeTop[e]) continue;
+    const double sf = EdgeSign(m.eocSign[s]).times(invAreaCell1);
+    uint32_t bads = 0;
+    const SoftFactor fs = soft_factor(sf, bads);
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const double xl = lo[((int64_t)e * L + k) * T + t], xh = ho[((int64_t)e * L + k) * T + t];
+      uint32_t bad = bads;
+      double pl = soft_mul(xl, fs, bad), x = soft_mul(xh, fs, bad);
+      if (bad) pl = rare_product(sf, xl), x = rare_product(sf, xh);
+      td[t] += pl;
+      // flxIn += max(0, x), flxOut += min(0, x): one add into the sum the sign selects
+      const bool in = ieee_lt(0.0, x), out = ieee_lt(x, 0.0);
+      const double acc = (in ? fin[t] : fout[t]) + x;
+      fin[t] = in ? acc : fin[t];
+      fout[t] = out ? acc : fout[t];
     }
+  }
+  const double hc = h[i], hpi = live ? hProvInv[i] : 0.0;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const int64_t it = i * T + t;
+    tend[it] = td[t];
+    if (live) {
+      const double up = mul_int(mul_int(trc[t], hc) + mul_int(td[t], dt), hpi);
+      const double mxn = up + mul_int(mul_int(fin[t], dt), hpi);
+      const double mnn = up + mul_int(mul_int(fout[t], dt), hpi);
+      trMax[it] = mx[t];
+      trMin[it] = mn[t];
+      fin[t] = clamp_quotient(mx[t] - up, (mxn - up) + eps);
+      fout[t] = clamp_quotient(up - mn[t], (up - mnn) + eps);
+    }
+    flxIn[it] = fin[t];
+    flxOut[it] = fout[t];
   }
 }
 
-// apps/ocean/tasks/solve.cc:270-282: rescale anti-diffusive fluxes.
-__global__ void k_oc_fct_c(DMesh m, Lev L, int T, const double *__restrict__ flxIn,
-                           const double *__restrict__ flxOut, double *ho) {
+// apps/ocean/tasks/solve.cc:270-282: rescale anti-diffusive fluxes,
+// max(0, x) min(R-(c1), R+(c2)) + min(0, x) min(R+(c1), R-(c2)), whose factor the
+// sign of x selects.
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_fct_c(DMesh m, Lev L, const double *__restrict__ flxIn,
+                                                  const double *__restrict__ flxOut, double *ho) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
   int e, k;
   L.split(i, e, k);
   if (k >= m.maxLevelEdgeTop[e]) return;
   const int2 c = m.coe[e];
+  const int64_t i1 = ((int64_t)c.x * L + k) * T, i2 = ((int64_t)c.y * L + k) * T;
+#pragma unroll
   for (int t = 0; t < T; ++t) {
     const double x = ho[i * T + t];
-    const int64_t i1 = ((int64_t)c.x * L + k) * T + t, i2 = ((int64_t)c.y * L + k) * T + t;
-    const double a = flxIn[i2] < flxOut[i1] ? flxIn[i2] : flxOut[i1];
-    const double b = flxOut[i2] < flxIn[i1] ? flxOut[i2] : flxIn[i1];
-    ho[i * T + t] = ((0.0 < x) ? x : 0.0) * a + ((x < 0.0) ? x : 0.0) * b;
+    const bool pos = ieee_lt(0.0, x), neg = ieee_lt(x, 0.0);
+    const double r1 = pos ? flxOut[i1 + t] : flxIn[i1 + t], r2 = pos ? flxIn[i2 + t] : flxOut[i2 + t];
+    const double r = ieee_lt(r2, r1) ? r2 : r1;
+    // (r as the first operand: it is often zero)
+    ho[i * T + t] = pos || neg ? mul_int(r, x) : 0.0;
   }
 }
 
 // apps/ocean/tasks/solve.cc:287-326
-__global__ void k_oc_accumulate_fct(DMesh m, Lev L, int T, const double *__restrict__ hProvInv,
-                                    const double *__restrict__ h, const double *__restrict__ ho,
-                                    const double *__restrict__ tr, double *trProv, double *tend,
-                                    double dt) {
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_accumulate_fct(DMesh m, Lev L, const double *__restrict__ hProvInv,
+                                                           const double *__restrict__ h,
+                                                           const double *__restrict__ ho,
+                                                           const double *__restrict__ tr, double *trProv,
+                                                           double *tend, double dt) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
   int c, k;
   L.split(i, c, k);
-  const double invAreaCell1 = 1.0 / m.areaCell[c];
+  const double invAreaCell1 = m.invAreaCell[c];
   const int n = m.nEoC[c];
-  for (int t = 0; t < T; ++t) {
-    double td = tend[i * T + t];
-    for (int j = 0; j < n; ++j) {
-      const int e = m.eoc[(int64_t)j * m.nC + c];
-      if (k < m.maxLevelEdgeTop[e])
-        td += m.eocSign[(int64_t)j * m.nC + c] * invAreaCell1 * ho[((int64_t)e * L + k) * T + t];
+  double td[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) td[t] = tend[i * T + t];
+  for (int j = 0; j < n; ++j) {
+    const int64_t s = (int64_t)j * m.nC + c;
+    const int e = m.eoc[s];
+    if (k >= m.maxLevelEdgeTop[e]) continue;
+    const double sf = EdgeSign(m.eocSign[s]).times(invAreaCell1);
+    uint32_t bads = 0;
+    const SoftFactor fs = soft_factor(sf, bads);
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const double x = ho[((int64_t)e * L + k) * T + t];
+      uint32_t bad = bads;
+      double p = soft_mul(x, fs, bad);
+      if (bad) p = rare_product(sf, x);
+      td[t] += p;
     }
-    tend[i * T + t] = td;
-    if (k < m.maxLevelCell[c]) trProv[i * T + t] = (tr[i * T + t] * h[i] + dt * td) * hProvInv[i];
+  }
+  const bool live = k < m.maxLevelCell[c];
+  const double hc = h[i], hpi = live ? hProvInv[i] : 0.0;
+#pragma unroll
+  for (int t = 0; t < T; ++t) {
+    const int64_t it = i * T + t;
+    tend[it] = td[t];
+    if (live) trProv[it] = mul_int(mul_int(tr[it], hc) + mul_int(td[t], dt), hpi);
   }
 }
 
+// rho of apps/ocean/tasks/solve.cc:352, once per edge instead of in every
+// cell-level on either side
+__global__ void __launch_bounds__(TPB) k_oc_hmix_rho(DMesh m, double coef, double *rho) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < m.nE) rho[e] = m.meshScalingDel2[e] * coef * m.dvEdge[e] / m.dcEdge[e];
+}
+
 // apps/ocean/tasks/solve.cc:328-366
-__global__ void k_oc_hmix(DMesh m, Lev L, int T, const double *__restrict__ hE,
-                          const double *__restrict__ tr, double *tend, double coef) {
+template <int T>
+__global__ void __launch_bounds__(TPB) k_oc_hmix(DMesh m, Lev L, const double *__restrict__ hE,
+                                                 const double *__restrict__ tr, const double *__restrict__ rho,
+                                                 double *tend) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
   int c, k;
   L.split(i, c, k);
-  const double invArea = 1.0 / m.areaCell[c];
+  const double invArea = m.invAreaCell[c];
   const int n = m.nEoC[c];
-  for (int t = 0; t < T; ++t) {
-    double td = tend[i * T + t];
-    for (int j = 0; j < n; ++j) {
-      const int e = m.eoc[(int64_t)j * m.nC + c];
-      if (k < m.maxLevelEdgeTop[e]) {
-        const int2 cc = m.coe[e];
-        const double rho = m.meshScalingDel2[e] * coef * m.dvEdge[e] / m.dcEdge[e];
-        const double ttf = tr[((int64_t)cc.y * L + k) * T + t] - tr[((int64_t)cc.x * L + k) * T + t];
-        const double flux = hE[(int64_t)e * L + k] * ttf * rho;
-        td -= m.eocSign[(int64_t)j * m.nC + c] * flux * invArea;
-      }
+  uint32_t bada = 0;
+  const SoftFactor fa = soft_factor(invArea, bada);
+  double td[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) td[t] = tend[i * T + t];
+  for (int j = 0; j < n; ++j) {
+    const int64_t s = (int64_t)j * m.nC + c;
+    const int e = m.eoc[s];
+    if (k >= m.maxLevelEdgeTop[e]) continue;
+    const int2 cc = m.coe[e];
+    const double he = hE[(int64_t)e * L + k], re = rho[e];
+    const EdgeSign sg(m.eocSign[s]);
+    uint32_t badm = bada;
+    const SoftFactor fh = soft_factor(he, badm), fr = soft_factor(re, badm);
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const double ttf = tr[((int64_t)cc.y * L + k) * T + t] - tr[((int64_t)cc.x * L + k) * T + t];
+      uint32_t bad = badm;
+      const double flux = soft_mul(soft_mul(ttf, fh, bad), fr, bad);
+      double x = soft_mul(sg.times(flux), fa, bad);
+      if (bad) x = rare_product(rare_product(sg.s, rare_product(rare_product(he, ttf), re)), invArea);
+      td[t] -= x;
     }
-    tend[i * T + t] = td;
   }
+#pragma unroll
+  for (int t = 0; t < T; ++t) tend[i * T + t] = td[t];
 }
 
 // apps/ocean/tasks/solve.cc:368-399
@@ -403,6 +529,21 @@ __global__ void k_oc_step_forward(int64_t n, const double *tend, const double *t
   if (i >= n) return;
   trNew[i] += w * tend[i];
   trPrev[i] = tr[i] + wsub * tend[i];
+}
+
+// Calls f with the tracer count as a compile-time constant.
+template <class F> void with_tracers(int T, F &&f) {
+  switch (T) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 3: f(std::integral_constant<int, 3>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    case 5: f(std::integral_constant<int, 5>{}); break;
+    case 6: f(std::integral_constant<int, 6>{}); break;
+    case 7: f(std::integral_constant<int, 7>{}); break;
+    case 8: f(std::integral_constant<int, 8>{}); break;
+    default: fail(MPASO_ERR_ARG, "ntr out of range (max 8)");
+  }
 }
 
 void check_levels(int L, int T) {
@@ -652,8 +793,10 @@ int mpaso_oc_calc_horiz_tracer_advection_flux_mono_low_order(
     const int olo = io.out(lowOrderFlux, MPASO_EDGES, L * T);
     io.stage();
     const DMesh &d = io.dm();
-    k_oc_low_order<<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, io.stream()>>>(d, L, T, io.ptr(intf),
-                                                                                 io.ptr(itr), io.ptr(olo));
+    with_tracers(T, [&](auto t) {
+      k_oc_low_order<t.value><<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, io.stream()>>>(
+          d, L, io.ptr(intf), io.ptr(itr), io.ptr(olo));
+    });
     io.finish();
   });
 }
@@ -670,8 +813,10 @@ int mpaso_oc_calc_horiz_tracer_advection_flux_mono_high_order(
     const int oho = io.out(highOrderFlux, MPASO_EDGES, L * T);
     io.stage();
     const DMesh &d = io.dm();
-    k_oc_high_order<<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, io.stream()>>>(d, L, T, io.ptr(intf),
-                                                                                  io.ptr(itr), io.ptr(oho));
+    with_tracers(T, [&](auto t) {
+      k_oc_high_order<t.value><<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, io.stream()>>>(
+          d, L, io.ptr(intf), io.ptr(itr), io.ptr(oho));
+    });
     io.finish();
   });
 }
@@ -696,14 +841,15 @@ int mpaso_oc_correct_and_rescale_high_order_mono_horiz_flux(
     io.stage();
     const DMesh &d = io.dm();
     const cudaStream_t s = io.stream();
-    k_oc_fct_a<<<blocks_for(((int64_t)d.nC + d.nE) * L, TPB), TPB, 0, s>>>(
-        d, L, T, io.ptr(intf), io.ptr(ilo), io.ptr(itr), io.ptr(oho), io.ptr(ofi), io.ptr(ofo),
-        io.ptr(omx), io.ptr(omn));
-    k_oc_fct_b<<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, s>>>(
-        d, L, T, io.ptr(ihpi), io.ptr(ih), io.ptr(ilo), io.ptr(itr), io.ptr(oho), io.ptr(ofi),
-        io.ptr(ofo), io.ptr(ote), io.ptr(omx), io.ptr(omn), dt);
-    k_oc_fct_c<<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, s>>>(d, L, T, io.ptr(ofi), io.ptr(ofo),
-                                                                   io.ptr(oho));
+    with_tracers(T, [&](auto t) {
+      k_oc_fct_a<t.value><<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, s>>>(d, L, io.ptr(intf), io.ptr(ilo),
+                                                                            io.ptr(itr), io.ptr(oho));
+      k_oc_fct_b<t.value><<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, s>>>(
+          d, L, io.ptr(ihpi), io.ptr(ih), io.ptr(ilo), io.ptr(itr), io.ptr(oho), io.ptr(ofi), io.ptr(ofo),
+          io.ptr(ote), io.ptr(omx), io.ptr(omn), dt);
+      k_oc_fct_c<t.value><<<blocks_for((int64_t)d.nE * L, TPB), TPB, 0, s>>>(d, L, io.ptr(ofi), io.ptr(ofo),
+                                                                            io.ptr(oho));
+    });
     io.finish();
   });
 }
@@ -722,8 +868,10 @@ int mpaso_oc_accumulate_horiz_tracer_advection_tend_mono_FCT(
     const int otp = io.out(tracersProv, MPASO_CELLS, L * T), ote = io.out(tend, MPASO_CELLS, L * T);
     io.stage();
     const DMesh &d = io.dm();
-    k_oc_accumulate_fct<<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, io.stream()>>>(
-        d, L, T, io.ptr(ihpi), io.ptr(ih), io.ptr(iho), io.ptr(itr), io.ptr(otp), io.ptr(ote), dt);
+    with_tracers(T, [&](auto t) {
+      k_oc_accumulate_fct<t.value><<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, io.stream()>>>(
+          d, L, io.ptr(ihpi), io.ptr(ih), io.ptr(iho), io.ptr(itr), io.ptr(otp), io.ptr(ote), dt);
+    });
     io.finish();
   });
 }
@@ -737,10 +885,14 @@ int mpaso_oc_tracer_hmix_del2_tend(mpaso_mesh m, int32_t nlev, int32_t ntr,
     const int L = nlev, T = ntr;
     const int ihe = io.in(layerThicknessEdge, MPASO_EDGES, L), itr = io.in(tracers, MPASO_CELLS, L * T);
     const int ote = io.out(tend, MPASO_CELLS, L * T);
+    const int rho = io.work(MPASO_EDGES, 1);
     io.stage();
     const DMesh &d = io.dm();
-    k_oc_hmix<<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, io.stream()>>>(d, L, T, io.ptr(ihe),
-                                                                            io.ptr(itr), io.ptr(ote), coef);
+    k_oc_hmix_rho<<<blocks_for(d.nE, TPB), TPB, 0, io.stream()>>>(d, coef, io.ptr(rho));
+    with_tracers(T, [&](auto t) {
+      k_oc_hmix<t.value><<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, io.stream()>>>(
+          d, L, io.ptr(ihe), io.ptr(itr), io.ptr(rho), io.ptr(ote));
+    });
     io.finish();
   });
 }

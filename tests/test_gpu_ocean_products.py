@@ -37,3 +37,44 @@ def test_ocean_step_at_the_window_of_the_integer_products(exp2, spec, ntr):
     got = st.get(G.FIELD_TRACERS)
     assert np.isfinite(want).all()
     assert np.array_equal(got, np.asarray(want).reshape(got.shape))
+
+
+@pytest.mark.parametrize("ntr", [1, 3, 4])
+@pytest.mark.parametrize("exp2", [-1060, -300, 0, 300])
+def test_ocean_tasks_at_the_window_of_the_integer_products(exp2, ntr):
+    """The same through the per-task entries, on columns of uneven depth."""
+    import mpaso.gpu as G
+    mesh = mpaso.Mesh.icosa(2)
+    L, T, dt = 4, ntr, 100.0
+    maxlev = np.random.default_rng(1).integers(1, L + 1, mesh.nCells).astype(np.int32)
+    f = fct_statics(mesh, L, maxLevelCell=maxlev)
+    h, hE, u, _ = ocean_state(mesh, 4, L, ntr)
+    rng = np.random.default_rng(8)
+    nC, nE = mesh.nCells, mesh.nEdges
+    tr = np.ldexp(rng.uniform(-1.0, 1.0, (nC, L, T)), exp2)
+    tr[rng.uniform(size=tr.shape) < 0.2] = 0.0
+    u[rng.uniform(size=u.shape) < 0.1] = 0.0
+    z = lambda *s: np.zeros(s)  # noqa: E731
+    a = dict(ntf=u * hE, hp=z(nC, L), hpi=z(nC, L), hni=z(nC, L), lo=z(nE, L, T), ho=z(nE, L, T), fi=z(nC, L, T),
+             fo=z(nC, L, T), tend=z(nC, L, T), mx=z(nC, L, T), mn=z(nC, L, T), tp=z(nC, L, T))
+    b = {k: v.copy() for k, v in a.items()}
+    dm = G.DeviceMesh(mesh, fct=f)
+    S = Oracle("restatement")
+    om, st, cfg = S.mesh(mesh), S.static(mesh, f), S.config(L, T)
+    dm.call("oc_calc_provisional_layer_thicknesses", L, h, a["ntf"], a["hp"], a["hpi"], a["hni"], dt)
+    dm.call("oc_calc_horiz_tracer_advection_flux_mono_low_order", L, T, a["ntf"], tr, a["lo"])
+    dm.call("oc_calc_horiz_tracer_advection_flux_mono_high_order", L, T, a["ntf"], tr, a["ho"])
+    dm.call("oc_correct_and_rescale_high_order_mono_horiz_flux", L, T, a["hpi"], h, a["ntf"], a["lo"], tr, a["ho"],
+            a["fi"], a["fo"], a["tend"], a["mx"], a["mn"], dt)
+    dm.call("oc_accumulate_horiz_tracer_advection_tend_mono_FCT", L, T, a["hpi"], h, a["ho"], tr, a["tp"], a["tend"],
+            dt)
+    dm.call("oc_tracer_hmix_del2_tend", L, T, hE, tr, a["tend"], 1e4)
+    S.call("oc_provisional_layer_thicknesses", om, st, cfg, h, b["ntf"], b["hp"], b["hp"], b["hpi"], b["hni"], dt)
+    S.call("oc_low_order", om, st, cfg, b["ntf"], tr, b["lo"])
+    S.call("oc_high_order", om, st, cfg, b["ntf"], tr, b["ho"])
+    S.call("oc_correct_and_rescale", om, st, cfg, b["hpi"], h, b["ntf"], b["lo"], tr, b["ho"], b["fi"], b["fo"],
+           b["tend"], b["mx"], b["mn"], dt)
+    S.call("oc_accumulate_fct", om, st, cfg, b["hpi"], h, b["ho"], tr, b["tp"], b["tend"], dt)
+    S.call("oc_hmix_del2", om, st, cfg, hE, tr, b["tend"], 1e4)
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
