@@ -4,21 +4,35 @@
 
 namespace mpaso {
 
-__global__ void k_gather_rows(const double *__restrict__ src, double *__restrict__ dst,
-                              const int32_t *__restrict__ perm, int64_t n, int row) {
+// Rows between the two numberings: dst[i] = src[perm[i]] or, SCATTER,
+// dst[perm[i]] = src[i], a thread an element of V (two doubles where the row
+// length and both addresses allow).
+template <bool SCATTER, class V>
+__global__ void __launch_bounds__(256) k_rows(const V *__restrict__ src, V *__restrict__ dst,
+                                              const int32_t *__restrict__ perm, int64_t total, Lev row) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n * row) return;
-  const int64_t e = i / row, r = i - e * row;
-  dst[i] = src[(int64_t)perm[e] * row + r];
+  if (i >= total) return;
+  int e, r;
+  row.split(i, e, r);
+  const int64_t j = (int64_t)perm[e] * row + r;
+  if constexpr (SCATTER)
+    dst[j] = src[i];
+  else
+    dst[i] = src[j];
 }
 
-__global__ void k_scatter_rows(const double *__restrict__ src, double *__restrict__ dst,
-                               const int32_t *__restrict__ perm, int64_t n, int row) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n * row) return;
-  const int64_t e = i / row, r = i - e * row;
-  dst[(int64_t)perm[e] * row + r] = src[i];
+namespace {
+template <bool SCATTER>
+void launch_rows(const double *src, double *dst, const int32_t *perm, int64_t n, int row, cudaStream_t s) {
+  const int64_t total = n * row;
+  if (row % 2 == 0 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
+    k_rows<SCATTER><<<blocks_for(total / 2, 256), 256, 0, s>>>((const double2 *)src, (double2 *)dst, perm, total / 2,
+                                                               row / 2);
+  else
+    k_rows<SCATTER><<<blocks_for(total, 256), 256, 0, s>>>(src, dst, perm, total, row);
+  MPASO_CUDA(cudaGetLastError());
 }
+}  // namespace
 
 // Rows between page-locked host memory (reference order, read or written
 // through its device alias) and device memory (context order), in one pass:
@@ -28,11 +42,12 @@ __global__ void k_scatter_rows(const double *__restrict__ src, double *__restric
 // export: dst[j] = src[iperm[j]] (rows of `row` doubles).
 template <bool IMPORT>
 __global__ void k_host_rows(const double *__restrict__ src, double *__restrict__ dst,
-                            const int32_t *__restrict__ iperm, int64_t n, int row, bool pairs) {
+                            const int32_t *__restrict__ iperm, int64_t n, Lev row, bool pairs) {
   const int64_t total = n * row, stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   auto dev = [&](int64_t i) {
-    const int64_t j = i / row, r = i - j * row;
+    int j, r;
+    row.split(i, j, r);
     return (int64_t)iperm[j] * row + r;
   };
   if (pairs) {  // total even, host side 16-byte aligned
@@ -72,14 +87,12 @@ void host_rows_pub(bool import, const double *src, double *dst, const int32_t *i
 
 void k_gather_rows_pub(const double *src, double *dst, const int32_t *perm, int64_t n, int row,
                        cudaStream_t s) {
-  k_gather_rows<<<blocks_for(n * row, 256), 256, 0, s>>>(src, dst, perm, n, row);
-  MPASO_CUDA(cudaGetLastError());
+  launch_rows<false>(src, dst, perm, n, row, s);
 }
 
 void k_scatter_rows_pub(const double *src, double *dst, const int32_t *perm, int64_t n, int row,
                         cudaStream_t s) {
-  k_scatter_rows<<<blocks_for(n * row, 256), 256, 0, s>>>(src, dst, perm, n, row);
-  MPASO_CUDA(cudaGetLastError());
+  launch_rows<true>(src, dst, perm, n, row, s);
 }
 
 bool is_device_pointer(const void *p) {

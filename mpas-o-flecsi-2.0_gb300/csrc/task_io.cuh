@@ -7,11 +7,6 @@
 
 namespace mpaso {
 
-__global__ void k_gather_rows(const double *__restrict__ src, double *__restrict__ dst,
-                              const int32_t *__restrict__ perm, int64_t n, int row);
-__global__ void k_scatter_rows(const double *__restrict__ src, double *__restrict__ dst,
-                               const int32_t *__restrict__ perm, int64_t n, int row);
-
 bool is_device_pointer(const void *p);
 // One pass between a page-locked host array (reference order, through its
 // device alias) and a device array (context order): import (host -> device)
