@@ -29,8 +29,10 @@
 // The FP64 pipe bounds these kernels (82-84% busy with every product and sum on
 // it, the issue slots 10-24%), so the products run on the integer pipe
 // (softmul.cuh, the same rounding bit for bit) and only the sums on the FP64
-// pipe.  Level-6 sphere, 60 levels x 3 tracers, per launch: oc_edges 1384 ->
-// 651 us (FP64 65% busy, integer 63%), oc_cells 659 -> 453, oc_final 484 -> 363.
+// pipe.  Level-6 sphere, 60 levels x 3 tracers, us per launch: oc_edges 1384 ->
+// 630 (FP64, ALU and issue each 62-66% busy), oc_cells 659 -> 399, oc_final 484 ->
+// 356 (451 and 363 with a branch to the hardware product after each slot; their
+// registers are capped at 80 and 64, uncapped 448 and 371).
 #include "rk4.cuh"
 #include "softmul.cuh"
 
@@ -106,8 +108,6 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
     uint32_t badw = 0;
     const SoftFactor fw = soft_factor(wgt, badw);
     double flx[T];
-#pragma unroll
-    for (int t = 0; t < T; ++t) flx[t] = 0.0;
     const int na = NA > 0 ? NA : m.maxAdv;
 #pragma unroll
     for (int a = 0; a < na; ++a) {
@@ -127,8 +127,9 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
 #pragma unroll
         for (int t = 0; t < T; ++t) p[t] = product_outside(tr[t], wx);
       }
+      // the first term is the sum's start (0 + x = x)
 #pragma unroll
-      for (int t = 0; t < T; ++t) flx[t] += p[t];
+      for (int t = 0; t < T; ++t) flx[t] = a ? flx[t] + p[t] : p[t];
     }
     const double dv = m.dvEdge[e];
     // LO = dv (max(0, f) tr1 + min(0, f) tr2): one of the two products is a zero
@@ -168,20 +169,48 @@ __global__ void __launch_bounds__(TPB) k_oc_edges(DMesh m, DStat st, Stage S, in
   }
 }
 
+// The cell kernels form the products of a whole item without a branch between
+// them, so that its loads and sums overlap; where one lay outside the integer
+// products' window (softmul.cuh) the item's sums are formed again by these calls.
+// (In K1, whose integer work already equals its FP64 work, zero factors would
+// have to be handled in line for that: 627 -> 666 us.)
+__device__ __noinline__ double product3_outside(double a, double b, double c) { return a * b * c; }
+
+// K2's sums over a cell's edges in hardware products.
+struct CellSums {
+  double td, fi, fo;
+};
+__device__ __noinline__ CellSums cell_sums_outside(const int *eoc, const double *sign, const double *LO,
+                                                   const double *A, int nC, int c, int n, int64_t off, int64_t row,
+                                                   double inva) {
+  CellSums r{0.0, 0.0, 0.0};
+  for (int j = 0; j < n; ++j) {
+    const int64_t s = (int64_t)j * nC + c, ie = eoc[s] * row + off;
+    const long long sm = sign_mask(sign[s]);
+    r.td += dflip(inva * LO[ie], sm);
+    const double ax = dflip(inva * A[ie], sm);
+    if (dgt0(ax))
+      r.fi += ax;
+    else
+      r.fo += ax;
+  }
+  return r;
+}
+
 // K2: per cell-level, for every tracer, the bounds over the cell and its
 // neighbours (solve.cc:194-214), the upwind tendency and flxIn / flxOut over
 // the cell's edges (solve.cc:232-249) and the limiter factors R+ / R-
 // (solve.cc:251-265).  Writes R2 = {R+, R-} and tLO = the upwind tendency
 // (divided by the area, as the reference's tend holds it).
 template <int T, int NC>
-__global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
+__global__ void __launch_bounds__(TPB, 3) k_oc_cells(DMesh m, Stage S, int L) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L || !S.fct) return;
   const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
   const int n = m.nEoC[c];
   const double invAreaCell1 = m.invAreaCell[c];  // 1 / areaCell
-  uint32_t bada = 0;
-  const SoftFactor fa = soft_factor(invAreaCell1, bada);
+  uint32_t bad = 0;
+  const SoftFactor fa = soft_factor(invAreaCell1, bad);
   double trc[T], mx[T], mn[T], td[T], fi[T], fo[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) {
@@ -191,42 +220,81 @@ __global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
   for_slots<NC>(n, [&](int j, bool ok) {
     const int64_t s = (int64_t)j * m.nC + c;
     const int64_t in0 = ((int64_t)m.coc[s] * L + k) * T;  // pads: the cell itself
-    const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;
+    const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;  // pads: slot 0, masked
     const long long sm = sign_mask(m.eocSign[s]);  // signedFactor = +-invAreaCell1
 #pragma unroll
     for (int t = 0; t < T; ++t) {
       const double x = S.tr_in[in0 + t];
       mx[t] = dmax(mx[t], x);
       mn[t] = dmin(mn[t], x);
-      if (ok) {
-        const double lo = S.LO[ie0 + t], ho = S.A[ie0 + t];
-        uint32_t bad = bada;
-        double pl = soft_mul(lo, fa, bad), pa = soft_mul(ho, fa, bad);
-        if (bad) pl = product_outside(invAreaCell1, lo), pa = product_outside(invAreaCell1, ho);
-        td[t] += dflip(pl, sm);
-        const double ax = dflip(pa, sm);
-        // flxIn += max(0, ax), flxOut += min(0, ax): one add into the sum the
-        // sign selects (integer-pipe selects; a zero ax changes neither sum,
-        // so none is kept), instead of an add in each of two divergent branches
-        const bool in = dgt0(ax), out = dlt0(ax);
-        const double acc = (in ? fi[t] : fo[t]) + ax;
+      const double pl = dflip(soft_mul(dmask(S.LO[ie0 + t], ok), fa, bad), sm);
+      const double ax = dflip(soft_mul(dmask(S.A[ie0 + t], ok), fa, bad), sm);
+      // flxIn += max(0, ax), flxOut += min(0, ax): one add into the sum the
+      // sign selects (integer-pipe selects; a zero ax changes neither sum,
+      // so none is kept), instead of an add in each of two divergent branches
+      // (the first terms are the sums' starts)
+      const bool in = dgt0(ax), out = dlt0(ax);
+      if (j == 0) {
+        td[t] = pl;
+        fi[t] = in ? ax : 0.0;
+        fo[t] = out ? ax : 0.0;
+      } else {
+        td[t] += pl;
+        const double acc = opaque(in ? fi[t] : fo[t]) + ax;
         fi[t] = in ? acc : fi[t];
         fo[t] = out ? acc : fo[t];
       }
     }
   });
+  if (bad) {
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const CellSums r = cell_sums_outside(m.eoc, m.eocSign, S.LO, S.A, m.nC, c, n, (int64_t)k * T + t, (int64_t)L * T,
+                                           invAreaCell1);
+      td[t] = r.td, fi[t] = r.fi, fo[t] = r.fo;
+    }
+  }
   const double h = S.h_in[i], hpi = S.hpi[i], dt = S.dt;
   const double eps = 1.e-10;
+  uint32_t badh = 0;
+  const SoftFactor fh = soft_factor(h, badh), fp = soft_factor(hpi, badh), fdt = soft_factor(dt, badh);
 #pragma unroll
   for (int t = 0; t < T; ++t) {
-    const double up = mul_int(mul_int(trc[t], h) + mul_int(td[t], dt), hpi);  // tracerUpwindNew
-    const double mxn = up + mul_int(mul_int(fi[t], dt), hpi);                 // tracerMaxNew
-    const double mnn = up + mul_int(mul_int(fo[t], dt), hpi);                 // tracerMinNew
+    // tracerUpwindNew, and what tracerMaxNew / tracerMinNew add to it
+    uint32_t out = badh;
+    double up = soft_mul(soft_mul(trc[t], fh, out) + soft_mul(td[t], fdt, out), fp, out);
+    double di = soft_mul(soft_mul(fi[t], fdt, out), fp, out), dn = soft_mul(soft_mul(fo[t], fdt, out), fp, out);
+    if (out) {
+      up = product_outside(product_outside(trc[t], h) + product_outside(dt, td[t]), hpi);
+      di = product3_outside(dt, fi[t], hpi), dn = product3_outside(dt, fo[t], hpi);
+    }
+    const double mxn = up + di, mnn = up + dn;
     const double rp = clamp_quotient(mx[t] - up, (mxn - up) + eps);
     const double rm = clamp_quotient(up - mn[t], (up - mnn) + eps);
     S.R2[i * T + t] = make_double2(rp, rm);
     S.tLO[i * T + t] = td[t];
   }
+}
+
+// K3's tendency in hardware products: the upwind part td plus the limited fluxes
+// (A null: none) minus the del2 fluxes (DF null: none) of a cell's edges.
+__device__ __noinline__ double cell_tend_outside(const int *eoc, const int *nbr, const double *sign, const double *A,
+                                                 const double2 *R2, const double *DF, int nC, int c, int n,
+                                                 int64_t off, int64_t row, double2 own, double inva, double td) {
+  for (int j = 0; A && j < n; ++j) {
+    const int64_t s = (int64_t)j * nC + c;
+    const int nb = nbr[s];
+    const double a = A[eoc[s] * row + off];
+    const double2 o = R2[(nb >> 1) * row + off];
+    const double2 r1 = nb & 1 ? own : o, r2 = nb & 1 ? o : own;
+    const double r = dgt0(a) ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
+    td += dflip(inva * ((dgt0(a) || dlt0(a) ? a : 0.0) * r), sign_mask(sign[s]));
+  }
+  for (int j = 0; DF && j < n; ++j) {
+    const int64_t s = (int64_t)j * nC + c;
+    td -= dflip(DF[eoc[s] * row + off] * inva, sign_mask(sign[s]));
+  }
+  return td;
 }
 
 // K3: per cell-level, for every tracer, the tendency: the upwind part, the
@@ -236,14 +304,12 @@ __global__ void __launch_bounds__(TPB) k_oc_cells(DMesh m, Stage S, int L) {
 // max(0, A) min(R-(c1), R+(c2)) + min(0, A) min(R+(c1), R-(c2)) with
 // (c1, c2) = cells(e), is A times the one minimum its sign selects.
 template <int T, int NC>
-__global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
+__global__ void __launch_bounds__(TPB, 4) k_oc_final(DMesh m, Stage S, int L) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nC * L) return;
   const int c = (int)(i / L), k = (int)(i - (int64_t)c * L);
   const int n = m.nEoC[c];
   const double invAreaCell1 = m.invAreaCell[c];
-  uint32_t bada = 0;
-  const SoftFactor fa = soft_factor(invAreaCell1, bada);
   double td[T];
   double2 own[T];
 #pragma unroll
@@ -251,9 +317,10 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
     td[t] = S.fct ? S.tLO[i * T + t] : 0.0;
     if (S.fct) own[t] = S.R2[i * T + t];
   }
+  uint32_t bad = 0;
+  const SoftFactor fa = soft_factor(invAreaCell1, bad);
   if (S.fct) {
     for_slots<NC>(n, [&](int j, bool ok) {
-      if (!ok) return;
       const int64_t s = (int64_t)j * m.nC + c;
       const long long sm = sign_mask(m.eocSign[s]);
       const int nb = m.nbr[s];
@@ -261,39 +328,36 @@ __global__ void __launch_bounds__(TPB) k_oc_final(DMesh m, Stage S, int L) {
       const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T, jn = ((int64_t)(nb >> 1) * L + k) * T;
 #pragma unroll
       for (int t = 0; t < T; ++t) {
-        const double a = S.A[ie0 + t];
+        const double a = dmask(S.A[ie0 + t], ok);
         const double2 o = S.R2[jn + t];
         const double2 r1 = first ? own[t] : o, r2 = first ? o : own[t];  // {R+, R-} of c1, c2
         // one product with the minimum the sign selects (integer-pipe selects);
         // a zero flux enters as +0, whose products are the +0 the reference's
         // max(0, A) / min(0, A) terms give
+        // (a zero factor -- local extrema -- makes the flux the zero, the other 1)
         const bool pos = dgt0(a);
         const double rmin = pos ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
-        // (a zero factor -- local extrema -- makes the flux the zero, the other 1)
         const bool some = dgt0(rmin);
         const double a0 = some && (pos || dlt0(a)) ? a : 0.0, r0 = some ? rmin : 1.0;
-        uint32_t bad = bada;
-        double x = soft_mul(soft_mul(a0, soft_factor(r0, bad), bad), fa, bad);
-        if (bad) x = product_outside(invAreaCell1, product_outside(a0, r0));
-        td[t] += dflip(x, sm);
+        td[t] += dflip(soft_mul(soft_mul(a0, soft_factor(r0, bad), bad), fa, bad), sm);
       }
     });
   }
   if (S.hmix) {
     for_slots<NC>(n, [&](int j, bool ok) {
-      if (!ok) return;
       const int64_t s = (int64_t)j * m.nC + c;
       const long long sm = sign_mask(m.eocSign[s]);
       const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const double d = S.DF[ie0 + t];
-        uint32_t bad = bada;
-        double x = soft_mul(d, fa, bad);
-        if (bad) x = product_outside(d, invAreaCell1);
-        td[t] -= dflip(x, sm);
-      }
+      for (int t = 0; t < T; ++t) td[t] -= dflip(soft_mul(dmask(S.DF[ie0 + t], ok), fa, bad), sm);
     });
+  }
+  if (bad) {
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+      td[t] = cell_tend_outside(m.eoc, m.nbr, m.eocSign, S.fct ? S.A : nullptr, S.R2, S.hmix ? S.DF : nullptr, m.nC, c,
+                                n, (int64_t)k * T + t, (int64_t)L * T, S.fct ? own[t] : make_double2(0.0, 0.0),
+                                invAreaCell1, S.fct ? S.tLO[i * T + t] : 0.0);
   }
 #pragma unroll
   for (int t = 0; t < T; ++t) {

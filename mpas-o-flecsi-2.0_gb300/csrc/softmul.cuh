@@ -8,19 +8,21 @@
 // four 32 x 32 -> 64 bit integer products, equal bit for bit to the hardware
 // product (1.3e9 random and special pairs), and leaves the FP64 pipe to the
 // sums.  Measured in SM cycles per warp instruction: DMUL and DADD 19.1 each,
-// soft_mul 12.0 alone (9.9 without the in-line zero), soft_mul with a DADD on
-// its result 19.2 against DMUL + DADD 38.2: the products cost nothing beside
-// the sums.  The ALU pipe bounds it; moving its shifts to multiplications
-// (14.7) or its additions to multiply-adds (13.1) was slower.
+// soft_mul about 12 alone, soft_mul with a DADD on its result 19.2 against DMUL +
+// DADD 38.2: the products cost nothing beside the sums.  The ALU pipe bounds it
+// (some 19 operations; the multiplications and one shift, as a product, run
+// beside it); more shifts as products (14.7) or additions as multiply-adds
+// (13.1) were slower.
 //
-// Both factors must have an exponent in [kSoftLo, kSoftLo + 512) (magnitudes
-// 2^-256 .. 2^256, so no product overflows or underflows); others -- subnormals,
-// infinities, NaN, a zero second factor -- set a bit of `bad` and the caller
-// takes product_outside() instead.  A zero first factor is common (tracer
-// plateaus, still water) and gives +0 in line: a branch that single lanes of
-// most warps take would make the warp issue the sums behind it twice, once
-// for each side.  The sign of such a zero is not kept; the sums it enters
-// start from +0 and cannot tell.
+// The second factor has an exponent in [kSoftLo, kSoftLo + 256) (magnitudes
+// 2^-128 .. 2^128: coefficients, fluxes, thicknesses) and the product one from
+// 2^-895 to 2^129, which leaves the first factor any normal number that a
+// decaying tracer tail runs through; others -- subnormals, infinities, NaN, the
+// rest -- set a bit of `bad` and the caller forms the products in hardware.  A
+// zero first factor is common (tracer plateaus, still water) and gives +0 in
+// line: a branch that single lanes of most warps take would make the warp issue
+// the sums behind it twice, once for each side.  The sign of such a zero is
+// not kept; the sums it enters start from +0 and cannot tell.
 #pragma once
 
 #include <cstdint>
@@ -29,35 +31,48 @@
 
 namespace mpaso {
 
-constexpr uint32_t kSoftLo = 767u << 20;       // lowest exponent, at its place in the high word
-constexpr uint32_t kSoftRange = 0x60000000u;   // set by exponents outside the window
+constexpr uint32_t kExp = 0x7ff00000u;     // exponent field of a high word
+constexpr uint32_t kSignExp = 0xfff00000u;
+constexpr uint32_t kSoftLo = 895u << 20;   // lowest exponent of a factor, at its place
+constexpr uint32_t kSoftMin = 128u << 20;  // lowest exponent of a product, likewise
+constexpr uint32_t kSoftOut = 0x40000000u; // set from 1024 exponents above that on, and by a borrow
 
 // A factor prepared once for several products: significand shifted up by 10
-// bits (so the cross products cannot overflow 64 bits), sign and exponent
-// relative to kSoftLo.
+// bits (so the cross products cannot overflow 64 bits), and sign and exponent
+// fields less the bias and kSoftMin (two sign bits add to the product's).
 struct SoftFactor {
   uint32_t h, l, x;
 };
-
-// `x` of a factor: sign and exponent fields relative to the window's start.
-// An exponent outside it borrows into or reaches bits 29 and 30.
-__device__ __forceinline__ uint32_t soft_exp(uint32_t hi) { return (hi & 0xfff00000u) - kSoftLo; }
+// The words of a double, hidden from the optimiser, which would turn tests of
+// them back into floating-point comparisons on the FP64 pipe.
+__device__ __forceinline__ void soft_words(double x, uint32_t &hi, uint32_t &lo) {
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+}
+// Likewise for a selected operand of one sum, which it would split into two.
+__device__ __forceinline__ double opaque(double x) {
+  asm("" : "+d"(x));
+  return x;
+}
 
 __device__ __forceinline__ SoftFactor soft_factor(double b, uint32_t &bad) {
-  const uint32_t hi = (uint32_t)__double2hiint(b), lo = (uint32_t)__double2loint(b);
+  uint32_t hi, lo;
+  soft_words(b, hi, lo);
   SoftFactor f;
   f.h = (__funnelshift_l(lo, hi, 10) & 0x3fffffffu) | 0x40000000u;
   f.l = lo << 10;
-  f.x = soft_exp(hi);
-  bad |= f.x & kSoftRange;
+  f.x = (hi & kSignExp) - (1023u << 20) - kSoftMin;
+  bad |= ((hi & kExp) - kSoftLo) & 0xf0000000u;  // an exponent outside borrows into or reaches these bits
   return f;
 }
 
 __device__ __forceinline__ double soft_mul(double a, const SoftFactor &f, uint32_t &bad) {
-  const uint32_t hi = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
-  const uint32_t x = soft_exp(hi);
+  uint32_t hi, al;
+  soft_words(a, hi, al);
   const bool zero = ((hi & 0x7fffffffu) | al) == 0;
-  bad |= zero ? 0u : x & kSoftRange;
+  // sign and exponent of the product less kSoftMin, valid below 1024.  With the
+  // factor's window a subnormal `a` stays below 0, an infinity or NaN above 1024.
+  const uint32_t x = (hi & kSignExp) + f.x;
+  bad |= zero ? 0u : x & kSoftOut;
   const uint32_t ah = (hi & 0xfffffu) | 0x100000u;
   // P = a f 2^10 = top 2^64 + lo(t2) 2^32 + lo(t0), in [2^114, 2^116)
   const uint64_t t0 = (uint64_t)al * f.l;
@@ -67,11 +82,12 @@ __device__ __forceinline__ double soft_mul(double a, const SoftFactor &f, uint32
   const uint32_t th = (uint32_t)(top >> 32), tl = (uint32_t)top, tr = (uint32_t)t2;
   const uint32_t n = th >> 19;  // 1 where the significands' product is >= 2
   const uint32_t s = 2 - n;     // brings the leading bit to the implicit bit's place
-  const uint32_t mh = __funnelshift_l(tl, th, s), ml = __funnelshift_l(tr, tl, s), r = tr << s;
+  const uint32_t mh = __funnelshift_l(tl, th, s), ml = __funnelshift_l(tr, tl, s), r = tr * (4 - 2 * n);
   // round to nearest even: r + 0x7fffffff + (odd | sticky) carries exactly when
   // the discarded part exceeds a half, or equals it and the result is odd
   const uint32_t inc = ((ml | min((uint32_t)t0, 1u)) & 1u) + 0x7fffffffu;
-  const uint32_t e = x + f.x + n * 0x100000u + ((2 * 767 - 1023 - 1) << 20);
+  // to add to the significand, whose leading bit counts one
+  const uint32_t e = x + (kSoftMin - (1u << 20)) + n * 0x100000u;
   uint32_t oh, ol;
   asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, %5, %6;\n\t}"
       : "=r"(ol), "=r"(oh)

@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_b(DMesh m, Lev L, const double *
       td[t] += pl;
       // flxIn += max(0, x), flxOut += min(0, x): one add into the sum the sign selects
       const bool in = ieee_lt(0.0, x), out = ieee_lt(x, 0.0);
-      const double acc = (in ? fin[t] : fout[t]) + x;
+      const double acc = opaque(in ? fin[t] : fout[t]) + x;
       fin[t] = in ? acc : fin[t];
       fout[t] = out ? acc : fout[t];
     }

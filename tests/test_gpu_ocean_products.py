@@ -1,7 +1,7 @@
-"""The ocean stage kernels' integer-pipe products at and outside their exponent
-window (magnitudes 2^-256 .. 2^256), against the oracle value for value: zeros,
-subnormals and factors on both sides of each end, one to three tracers, on
-stencils of exactly ten cells and of run-time width."""
+"""The ocean kernels' integer-pipe products at and outside their exponent windows
+(factors 2^-128 .. 2^128, products 2^-895 .. 2^129), against the oracle value
+for value: zeros, subnormals and values on both sides of each end, one to
+three tracers, on stencils of exactly ten cells and of run-time width."""
 import numpy as np
 import pytest
 
@@ -15,7 +15,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("ntr", [1, 2, 3])
 @pytest.mark.parametrize("spec", [("icosa", 2), ("hex", 9, 6)])
-@pytest.mark.parametrize("exp2", [-1060, -300, -257, -250, 0, 240, 300])
+@pytest.mark.parametrize("exp2", [-1060, -960, -920, -880, -300, -130, 0, 100, 125, 300])
 def test_ocean_step_at_the_window_of_the_integer_products(exp2, spec, ntr):
     import mpaso.gpu as G
     mesh = mpaso.Mesh.icosa(spec[1]) if spec[0] == "icosa" else mpaso.Mesh.hex(spec[1], spec[2], 20e3, 1e-4)
@@ -40,7 +40,7 @@ def test_ocean_step_at_the_window_of_the_integer_products(exp2, spec, ntr):
 
 
 @pytest.mark.parametrize("ntr", [1, 3, 4])
-@pytest.mark.parametrize("exp2", [-1060, -300, 0, 300])
+@pytest.mark.parametrize("exp2", [-1060, -900, -130, 0, 125, 300])
 def test_ocean_tasks_at_the_window_of_the_integer_products(exp2, ntr):
     """The same through the per-task entries, on columns of uneven depth."""
     import mpaso.gpu as G
