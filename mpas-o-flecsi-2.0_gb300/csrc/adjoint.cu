@@ -45,6 +45,7 @@
 #include <cstring>
 
 #include "rk4.cuh"
+#include "softmul.cuh"
 
 namespace mpaso {
 
@@ -400,7 +401,9 @@ template <int NL> __device__ __forceinline__ double lane_sum(double v) {
 // the upwind sum, flxIn / flxOut and hProv.  NL lanes per cell share its edge
 // slots; the bounds merge as (value, slot) with the lower slot (the cell
 // itself first) winning ties, which is the reference's sequential max / min.
-template <int NL, int NC>
+// OC: the ocean app, whose thickness and thickness flux are prescribed (their
+// cotangents are not formed).
+template <int NL, int NC, bool OC>
 __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L, int64_t g) {
   const int lane = (int)(g & (NL - 1));
   const int64_t i = g / NL;
@@ -426,7 +429,7 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L
       const double aa = a.A[((int64_t)m.eoc[s] * L + k) * T + t];
       const double sa = dmask(dflip(aa, sign_mask(m.eocSign[s])), ok);
       const bool in = dgt0(sa);
-      const double f = (in ? fi : fo) + sa;
+      const double f = opaque(in ? fi : fo) + sa;
       fi = in ? f : fi, fo = in ? fo : f;
       const double x = a.tr[((int64_t)m.coc[s] * L + k) * T + t];
       if (dkey(mx) < dkey(x)) mx = x, smx = j;
@@ -437,6 +440,7 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L
       const bool first = nb & 1;
       const int64_t jo = ((int64_t)(nb >> 1) * L + k) * T + t;
       const double2 ot = a.R2[jo];
+      const double go = a.gq[jo];
       int sel = 0;  // 1: R+ of this cell, 2: R- of this cell
       if (!ok)
         ;
@@ -445,9 +449,8 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L
       else if (dlt0(aa))
         sel = first ? (dkey(ot.y) < dkey(own.x) ? 0 : 1) : (dkey(own.y) < dkey(ot.x) ? 2 : 0);
       if (sel) {  // one subtraction and one fma into the factor's sum (selected operands)
-        const double go = a.gq[jo];
-        const double G = (first ? go : gc) - (first ? gc : go);  // g(c2) - g(c1)
-        const double acc = fma(G, aa, sel == 1 ? lrp : lrm);
+        const double G = opaque(first ? go : gc) - opaque(first ? gc : go);  // g(c2) - g(c1)
+        const double acc = fma(G, aa, opaque(sel == 1 ? lrp : lrm));
         lrp = sel == 1 ? acc : lrp;
         lrm = sel == 1 ? lrm : acc;
       }
@@ -468,7 +471,7 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L
     if (lane) continue;
     // upwind sum: area-weighted from the sw kernels, divided by the area (as
     // the reference's tend holds it) from the ocean kernels
-    const double num = fma(a.ocean ? a.dt : dtia, a.tLO[it], trc * hin);
+    const double num = fma(OC ? a.dt : dtia, a.tLO[it], trc * hin);
     const double up = num * hpi;
     double lup = 0.0, ldp = 0.0, ldm = 0.0;
     double2 lb = make_double2(0.0, 0.0);  // cotangents of the max / min bounds
@@ -488,22 +491,24 @@ __device__ __forceinline__ void tr_a_item(const DMesh &m, const TrArgs &a, Lev L
     a.ltl[it] = lup * dthi;
     a.lmm[it] = lb;
     a.amm[it] = make_int2(smx < 0 ? c : m.coc[(int64_t)smx * m.nC + c], smn < 0 ? c : m.coc[(int64_t)smn * m.nC + c]);
-    lh = fma(lup * trc, hpi, lh);
-    lhpi = fma(lup, num, lhpi);
-    lhpi = fma(fma(ldp, fi, -ldm * fo), dtia, lhpi);
+    if constexpr (!OC) {
+      lh = fma(lup * trc, hpi, lh);
+      lhpi = fma(lup, num, lhpi);
+      lhpi = fma(fma(ldp, fi, -ldm * fo), dtia, lhpi);
+    }
   }
-  if (lane || a.ocean) return;  // ocean: h and the thickness flux are prescribed
+  if (OC || lane) return;
   // hProv = h + dt tend_h: its cotangent goes to h and to the thickness tendency
   const double lhp = -lhpi * hpi * hpi;
   a.muh_t[i] = lh + lhp;
   a.lk_h[i] = fma(a.dt, lhp, a.lk_h[i]);
 }
 
-template <int NL, int NC>
-__global__ void __launch_bounds__(TPB) k_adj_tr_a(DMesh m, TrArgs a, Lev L) {
+template <int NL, int NC, bool OC>
+__global__ void __launch_bounds__(TPB, OC ? 4 : 1) k_adj_tr_a(DMesh m, TrArgs a, Lev L) {
   const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (g / NL >= (int64_t)m.nC * L) return;  // whole groups: all lanes of a live cell stay
-  tr_a_item<NL, NC>(m, a, L, g);
+  tr_a_item<NL, NC, OC>(m, a, L, g);
 }
 
 // B3 of this reversed stage with TA of the next one (the stage before it in the
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(TPB) k_adj_b3_tra(DMesh m, DStat st, AdjArgs a
   const int64_t nCL = (int64_t)m.nC * L;
   if (i < nCL) {
     b3_cell_item(m, a, L, i);
-    tr_a_item<1, NC>(m, tn, L, i);
+    tr_a_item<1, NC, false>(m, tn, L, i);
     return;
   }
   i -= nCL;
@@ -541,8 +546,8 @@ __device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, Lev L
   const int T = a.T;
   const int2 c = m.coe[e];
   const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
-  const double he = a.ocean ? a.hEx[i] : 0.5 * (a.h[i1] + a.h[i2]);
-  const double F = a.ocean ? a.Fx[i] : a.u[i] * he, dv = m.dvEdge[e];
+  const double he = 0.5 * (a.h[i1] + a.h[i2]);
+  const double F = a.u[i] * he, dv = m.dvEdge[e];
   const bool pos = dgt0(F), neg = dlt0(F);
   const int mask = a.fct ? m.hoMask[(int64_t)e * m.fctLev + k] : 0;
   const double kd = a.hmix ? a.kd[e] : 0.0;
@@ -563,7 +568,7 @@ __device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, Lev L
       if (ap || an) {
         const double2 r1 = a.R2[i1t], r2 = a.R2[i2t], f1 = a.lfio[i1t], f2 = a.lfio[i2t];
         const double rmin = ap ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
-        lA = fma(G, rmin, (ap ? f2.x : f2.y) - (ap ? f1.y : f1.x));
+        lA = fma(G, rmin, opaque(ap ? f2.x : f2.y) - opaque(ap ? f1.y : f1.x));
       }
       const double lLO = G + (a.ltl[i2t] - a.ltl[i1t]) - lA;
       if (pos || neg) {  // the upwind value's cotangent, on the side the flux sign picks
@@ -609,14 +614,73 @@ __device__ __forceinline__ void tr_b_item(const DMesh &m, const TrArgs &a, Lev L
   lF_out = lF, lhe_out = lhe;
 }
 
-__global__ void __launch_bounds__(TPB) k_adj_tr_b(DMesh m, TrArgs a, Lev L) {
+// TB for the ocean app: the flux's own cotangents are not formed, which leaves
+// per tracer six sums and six products, the latter on the integer pipe (level 5,
+// 20 levels x 3 tracers: TBNEW).
+__device__ __noinline__ double rare_centred_part(double dv, double lAF) { return 0.5 * dv * lAF; }
+
+__global__ void __launch_bounds__(TPB) k_adj_oc_tr_b(DMesh m, TrArgs a, Lev L) {
+  stage_prologue();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= (int64_t)m.nE * L) return;
-  double lF, lhe;
-  tr_b_item(m, a, L, i, lF, lhe);
-  if (a.ocean) return;
-  a.lFt[i] = lF;
-  a.lhet[i] = lhe;
+  int e, k;
+  L.split(i, e, k);
+  const int T = a.T;
+  const int2 c = m.coe[e];
+  const int64_t i1 = ((int64_t)c.x * L + k) * T, i2 = ((int64_t)c.y * L + k) * T;
+  const double he = a.hEx[i], F = a.Fx[i], dv = m.dvEdge[e], kd = a.hmix ? a.kd[e] : 0.0;
+  const bool pos = dgt0(F), neg = dlt0(F);
+  const int mask = a.fct ? m.hoMask[(int64_t)e * m.fctLev + k] : 0;
+  uint32_t badf = 0, badm = 0;
+  const SoftFactor fF = soft_factor(F, badf), fdv = soft_factor(dv, badf);
+  const SoftFactor fh = soft_factor(he, badm), fk = soft_factor(kd, badm);
+  for (int t = 0; t < T; ++t) {
+    const int64_t it = i * T + t, j1 = i1 + t, j2 = i2 + t;
+    const double G = a.gq[j2] - a.gq[j1];
+    double p1 = 0.0, p2 = 0.0;
+    if (a.fct) {
+      const double aa = a.A[it];
+      const double2 r1 = a.R2[j1], r2 = a.R2[j2], f1 = a.lfio[j1], f2 = a.lfio[j2];
+      const double l1 = a.ltl[j1], l2 = a.ltl[j2];
+      // the branch the flux sign took, as one subtraction and one fma whose
+      // operands the sign selects (integer-pipe selects)
+      const bool ap = dgt0(aa), an = dlt0(aa);
+      const double rmin = ap ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
+      const double lAx = fma(G, rmin, opaque(ap ? f2.x : f2.y) - opaque(ap ? f1.y : f1.x));
+      const double lA = ap || an ? lAx : 0.0;
+      const double lLO = G + (l2 - l1) - lA;
+      // the upwind value's cotangent, on the side the flux sign picks
+      uint32_t bad = badf;
+      double pq = soft_mul(soft_mul(lLO, fdv, bad), fF, bad), lAF = soft_mul(lA, fF, bad);
+      if (bad) pq = product_outside(product_outside(lLO, dv), F), lAF = product_outside(lA, F);
+      p1 = pos ? pq : 0.0;
+      p2 = pos || !neg ? 0.0 : pq;
+      if (!mask) {
+        const double q = rare_centred_part(dv, lAF);
+        p1 += q, p2 += q;
+      }
+      a.lho[it] = make_double2(mask && pos ? lAF : 0.0, mask && neg ? lAF : 0.0);
+    }
+    if (a.hmix) {  // tend -= inva sum sign DF, DF = h_e (tr2 - tr1) kd
+      uint32_t bad = badm;
+      double q = soft_mul(soft_mul(G, fh, bad), fk, bad);
+      if (bad) q = product_outside(product_outside(G, he), kd);
+      p1 += q, p2 -= q;
+    }
+    a.p12[it] = make_double2(p1, p2);
+  }
+}
+
+// What cell c receives of the bounds of its neighbour's cell-level-tracer `ot`,
+// held by the cells am: one add of the cotangent of the bound it holds (a
+// neighbour is above the cell or below it, never both).
+__device__ __forceinline__ double add_bounds(double lt, int2 am, const double2 *lmm, int64_t ot, int c) {
+  const bool hi = am.x == c;
+  if (hi || am.y == c) {
+    const double2 l = lmm[ot];
+    lt += opaque(hi ? l.x : l.y);
+  }
+  return lt;
 }
 
 // TC (cells): the tracer cotangent of the stage input, gathered from the
@@ -633,8 +697,8 @@ __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L
   int c, k;
   L.split(i, c, k);
   const int n = m.nEoC[c], T = a.T;
-  const double hinv = a.ocean ? 1.0 : rcp_nr(a.h[i]), inva = m.invAreaCell[c];
-  double mh = a.fct && !a.ocean ? a.muh_t[i] : 0.0;
+  const double hinv = rcp_nr(a.h[i]), inva = m.invAreaCell[c];
+  double mh = a.fct ? a.muh_t[i] : 0.0;
   for (int t = 0; t < T; ++t) {
     const int64_t it = i * T + t;
     double lt = 0.0;
@@ -646,9 +710,7 @@ __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L
         const int oc = m.cocU[s];
         if (oc >= 0) {
           const int64_t ot = ((int64_t)oc * L + k) * T + t;
-          const int2 ao = a.amm[ot];
-          if (ao.x == c) lt += a.lmm[ot].x;
-          if (ao.y == c) lt += a.lmm[ot].y;
+          lt = add_bounds(lt, a.amm[ot], a.lmm, ot, c);
         }
       }
     }
@@ -681,21 +743,79 @@ __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L
       if (am.x == c) lt += lb.x;
       if (am.y == c) lt += lb.y;
     }
-    const double mq = lt * hinv;  // sw: tr = q / h; ocean: the state is tr itself
-    if (!a.ocean) mh = fma(-mq, a.tr[it], mh);
+    const double mq = lt * hinv;  // tr = q / h
+    mh = fma(-mq, a.tr[it], mh);
     a.gq[it] = combine(a.rk, a.dt, it, mq, a.lam_q, a.acc_q, a.lk_q) * inva;
   }
   mh_out = mh;
   return lane == 0;
 }
 
-template <int NL>
-__global__ void __launch_bounds__(TPB) k_adj_tr_c(DMesh m, TrArgs a, Lev L) {
-  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (g / NL >= (int64_t)m.nC * L) return;  // whole groups: all lanes of a live cell stay
-  double mh;
-  if (tr_c_item<NL>(m, a, L, g, mh) && !a.ocean) a.muh_t[g / NL] = mh;
+// TC for the ocean app: the state is the tracer itself and thickness has no
+// cotangent.  TC tracers at a time share the indices and coefficients of the
+// gathers (a column of levels and tracers fills the GPU, so one lane a cell).
+template <int TC, int NC>
+__global__ void __launch_bounds__(TPB) k_adj_oc_tr_c(DMesh m, TrArgs a, Lev L) {
+  stage_prologue();
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= (int64_t)m.nC * L) return;
+  int c, k;
+  L.split(i, c, k);
+  const int n = m.nEoC[c], T = a.T;
+  const double inva = m.invAreaCell[c];
+  for (int t0 = 0; t0 < T; t0 += TC) {
+    double lt[TC];
+#pragma unroll
+    for (int t = 0; t < TC; ++t) lt[t] = 0.0;
+    for_slots<NC>(n, [&](int j, bool ok) {
+      const int64_t s = (int64_t)j * m.nC + c;
+      const int64_t ie = ((int64_t)m.eoc[s] * L + k) * T + t0;
+      const int side = (m.nbr[s] & 1) ^ 1;  // of cells(e), which this cell is
+      const int oc = a.fct ? m.cocU[s] : -1;
+#pragma unroll
+      for (int t = 0; t < TC; ++t) lt[t] += dmask(reinterpret_cast<const double *>(a.p12 + ie + t)[side], ok);
+      if (oc >= 0) {
+        const int64_t ot = ((int64_t)oc * L + k) * T + t0;
+#pragma unroll
+        for (int t = 0; t < TC; ++t) lt[t] = add_bounds(lt[t], a.amm[ot + t], a.lmm, ot + t, c);
+      }
+    });
+    if (a.fct)
+      for (int j0 = 0; j0 < m.maxAdvR; j0 += 4) {
+        int e[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) e[u] = j0 + u < m.maxAdvR ? m.advRe[(int64_t)(j0 + u) * m.nC + c] : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (e[u] < 0) continue;
+          const double2 w = m.advRc[(int64_t)(j0 + u) * m.nC + c];
+          const double2 *lh = a.lho + ((int64_t)e[u] * L + k) * T + t0;
+#pragma unroll
+          for (int t = 0; t < TC; ++t) {
+            // one of {F > 0 part, F < 0 part} is +0: pick the other with its coefficient
+            const double2 l = lh[t];
+            const bool p = dbits(l.x) != 0;
+            lt[t] = fma(p ? w.x : w.y, p ? l.x : l.y, lt[t]);
+          }
+        }
+        if (e[3] < 0) break;
+      }
+#pragma unroll
+    for (int t = 0; t < TC; ++t) {
+      const int64_t it = i * T + t0 + t;
+      if (a.fct) {
+        lt[t] += a.ltrs[it];
+        const int2 am = a.amm[it];
+        const double2 lb = a.lmm[it];
+        if (am.x == c) lt[t] += lb.x;
+        if (am.y == c) lt[t] += lb.y;
+      }
+      a.gq[it] = combine(a.rk, a.dt, it, lt[t], a.lam_q, a.acc_q, a.lk_q) * inva;
+    }
+  }
 }
+
+template <int TC> auto oc_tr_c_kernel(bool c6) { return c6 ? k_adj_oc_tr_c<TC, 6> : k_adj_oc_tr_c<TC, 0>; }
 
 // The sw app with tracers, fused by item: TB and B1 of one edge-level in one
 // thread (the tracer part's flux cotangents pass in registers) ...
@@ -890,10 +1010,10 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
     const TrArgs t = tr_args(s, A, rk, j);
     constexpr int NLA = 1, NLC = 2;  // lanes per cell (measured best at level 6)
     if (t.fct && !tra_done) {
-      if (m.maxEoC <= 6)
-        launch_pdl(k_adj_tr_a<NLA, 6>, nC * NLA, TPL, pdl, st, m, t, L);
-      else
-        launch_pdl(k_adj_tr_a<NLA, 0>, nC * NLA, TPL, pdl, st, m, t, L);
+      const bool c6 = m.maxEoC <= 6;
+      launch_pdl(ocean ? (c6 ? k_adj_tr_a<NLA, 6, true> : k_adj_tr_a<NLA, 0, true>)
+                       : (c6 ? k_adj_tr_a<NLA, 6, false> : k_adj_tr_a<NLA, 0, false>),
+                 nC * NLA, TPL, pdl, st, m, t, L);
     }
     // two lanes per cell-level hide gather latency on small meshes; with a
     // million cell-levels or more there is parallelism enough, and the
@@ -920,11 +1040,10 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
       launch_pdl(k_adj_b3, nC + nE, TPL, pdl, st, m, s.st, a, L);
       return false;
     }
-    launch_pdl(k_adj_tr_b, nE, TPL, pdl, st, m, t, L);
-    if (one_lane)
-      launch_pdl(k_adj_tr_c<1>, nC, TPL, pdl, st, m, t, L);
-    else
-      launch_pdl(k_adj_tr_c<NLC>, nC * NLC, TPL, pdl, st, m, t, L);
+    launch_pdl(k_adj_oc_tr_b, nE, TPL, pdl, st, m, t, L);
+    const bool c6 = m.maxEoC <= 6;
+    launch_pdl(s.T % 3 == 0 ? oc_tr_c_kernel<3>(c6) : s.T % 2 == 0 ? oc_tr_c_kernel<2>(c6) : oc_tr_c_kernel<1>(c6), nC,
+               TPL, pdl, st, m, t, L);
   }
   if (ocean) return false;  // the ocean's h and u are prescribed: nothing more to reverse
   if (m.maxEoE == 10)

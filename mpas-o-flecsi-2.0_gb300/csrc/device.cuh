@@ -171,6 +171,12 @@ __device__ __forceinline__ double dclamp01(double x) {
   const long long p = b > 0 ? b : 0LL;
   return bitsd(p > 0x3ff0000000000000LL ? 0x3ff0000000000000LL : p);
 }
+// Hides from the optimiser that a sum's operand was selected: it would form
+// the sum with either operand, on the FP64 pipe, and select afterwards.
+__device__ __forceinline__ double opaque(double x) {
+  asm("" : "+d"(x));
+  return x;
+}
 // x * s for s in {-1, +1} given as the sign bit mask (0 or 1<<63).
 __device__ __forceinline__ double dflip(double x, long long signmask) {
   return bitsd(dbits(x) ^ signmask);

@@ -378,7 +378,7 @@ __device__ __forceinline__ void cell_limiter(const DMesh &m, const Stage &S, Lev
       // the accumulator the sign selects (integer-pipe select, same sums)
       const double ax = dmask(dflip(S.A[ie0 + t], sm), ok);
       const bool in = dgt0(ax);
-      const double acc = (in ? fi[t] : fo[t]) + ax;
+      const double acc = opaque(in ? fi[t] : fo[t]) + ax;
       fi[t] = in ? acc : fi[t];
       fo[t] = in ? fo[t] : acc;
     }

@@ -48,12 +48,6 @@ struct SoftFactor {
 __device__ __forceinline__ void soft_words(double x, uint32_t &hi, uint32_t &lo) {
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
 }
-// Likewise for a selected operand of one sum, which it would split into two.
-__device__ __forceinline__ double opaque(double x) {
-  asm("" : "+d"(x));
-  return x;
-}
-
 __device__ __forceinline__ SoftFactor soft_factor(double b, uint32_t &bad) {
   uint32_t hi, lo;
   soft_words(b, hi, lo);
