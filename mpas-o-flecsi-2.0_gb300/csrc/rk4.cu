@@ -98,8 +98,7 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
   if (i < nEL * LANES) {
     const int lane = (int)(i & (LANES - 1));
     i /= LANES;
-    int e, k;
-    L.split(i, e, k);
+    const int e = (int)(i / (int)L), k = (int)(i - (int64_t)e * L);
     // q = sum_j W_j F_j (pv_e + pv_j) / 2 = (Pv_e sum W/8 F2_j + sum W/8 F2_j Pv_j)
     double s1 = 0.0, s2 = 0.0;
     const int ne = NW > 0 ? NW : m.maxEoE;
@@ -116,6 +115,7 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
     s2 = lane_total<LANES>(s2);
     if (lane) return;
     const double q = fma(S.pve[i], s1, s2);
+    if (S.tape_s1) S.tape_s1[i] = s1;
     const int2 c = m.coe[e];
     const int64_t i1 = (int64_t)c.x * L + k, i2 = (int64_t)c.y * L + k;
     // - (ke2 - ke1 + g (h2 + b2 - h1 - b1)) / dc + nu (div2 - div1) / dc, with the
@@ -128,15 +128,18 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
       const int2 v = m.voe[e];
       tend = fma(-st.nuDv[e], S.vort[(int64_t)v.y * L + k] - S.vort[(int64_t)v.x * L + k], tend);
     }
-    // every load before the first store (see the cells below)
-    const double up = S.u_prev[i], acc0 = S.stage == 0 ? up : S.u_acc[i];
-    const double acc = fma(S.w_acc, tend, acc0), out = S.pin_u ? up : fma(S.w_sub, tend, up);
-    if (S.tape_s1) S.tape_s1[i] = s1;
-    if (S.stage == 3) {
-      S.u_new[i] = S.pin_u ? up : acc;
-    } else {
-      S.u_out[i] = out;
-      S.u_acc[i] = acc;
+    const double up = S.u_prev[i];
+    switch (S.stage) {
+      case 0:
+        S.u_out[i] = S.pin_u ? up : fma(S.w_sub, tend, up);
+        S.u_acc[i] = fma(S.w_acc, tend, up);
+        break;
+      case 3:
+        S.u_new[i] = S.pin_u ? up : fma(S.w_acc, tend, S.u_acc[i]);
+        break;
+      default:
+        S.u_out[i] = S.pin_u ? up : fma(S.w_sub, tend, up);
+        S.u_acc[i] = fma(S.w_acc, tend, S.u_acc[i]);
     }
     if constexpr (SPLIT && T > 0)
       edge_tracer_fluxes<T, NW>(m, S, L, e, k, i, i1, i2, S.FG[i].x, h1 + h2, st.dvh, st.cpm2, st.kdh);
@@ -145,34 +148,48 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
   i -= nEL * LANES;
   if (i >= (int64_t)m.nC * L) return;
   constexpr int NC = NW > 0 ? 6 : 0;  // the unrolled variant also unrolls the cell loops
-  int c, k;
-  L.split(i, c, k);
+  const int c = (int)(i / (int)L), k = (int)(i - (int64_t)c * L);
   const int n = m.nEoC[c];
   double tend_h = 0.0;  // sum edgeSign dv F / area, from F2 with the halved weights (0 in pads)
   for_slots<NC>(n, [&](int j, bool) {
     const int64_t s = (int64_t)j * m.nC + c;
     tend_h = fma(st.sdvi[s], S.FG[(int64_t)m.eoc[s] * L + k].x, tend_h);
   });
-  // The stores come last: a load behind a store to memory it might alias waits
-  // for a round trip of its own, and on a mesh too small to fill the GPU those
-  // round trips are most of the kernel.
+  // The stores come behind the limiter's loads: a load behind a store to memory it
+  // might alias waits for a round trip of its own, and on a mesh too small to
+  // fill the GPU those round trips are most of the kernel (64 x 64 plane: 62 us per
+  // step with the stores ahead of the limiter, 56 so).  Held back further, behind
+  // the limiter's arithmetic, they cost registers (level 7, 3 tracers: 70 us per
+  // launch against 66).
   const double hp = S.h_prev[i], acc0 = S.stage == 0 ? hp : S.h_acc[i];
+  auto update_h = [&] {
+    const double acc = fma(S.w_acc, tend_h, acc0);
+    if (S.stage == 3) {
+      S.h_new[i] = acc;
+    } else {
+      S.h_out[i] = fma(S.w_sub, tend_h, hp);
+      S.h_acc[i] = acc;
+    }
+  };
   if constexpr (T > 0) {
+    if (!SPLIT && !S.fct) {  // (held back here the stores only cost registers: level 7, 3 levels, 97 -> 99)
+      update_h();
+      cell_upwind<T, NC>(m, S, L, c, k, i);
+      if (S.tape_hpi) S.tape_hpi[i] = 0.0;
+      return;
+    }
     // provisional thickness (apps/ocean/tasks/solve.cc:60-97): h + dt tend_h
     const double hin = S.h_in[i];
     const double hpi = S.fct ? rcp_nr(fma(S.dt, tend_h, hin)) : 0.0;
-    if constexpr (SPLIT)
+    if constexpr (SPLIT) {
+      update_h();
       S.hpw[i] = hpi;
-    else
-      cell_limiter<T, NC>(m, S, L, c, k, i, hin, hpi);
+    } else {
+      cell_limiter<T, NC>(m, S, L, c, k, i, hin, hpi, update_h);
+    }
     if (S.tape_hpi) S.tape_hpi[i] = hpi;
-  }
-  const double acc = fma(S.w_acc, tend_h, acc0);
-  if (S.stage == 3) {
-    S.h_new[i] = acc;
   } else {
-    S.h_out[i] = fma(S.w_sub, tend_h, hp);
-    S.h_acc[i] = acc;
+    update_h();
   }
 }
 
@@ -191,7 +208,10 @@ __global__ void MPASO_BOUNDS(OC) k_sw_limit(DMesh m, Stage S, Lev L) {
   if (i >= (int64_t)m.nC * L) return;
   int c, k;
   L.split(i, c, k);
-  cell_limiter<T, NC>(m, S, L, c, k, i, S.h_in[i], S.hpw[i]);
+  if (S.fct)
+    cell_limiter<T, NC>(m, S, L, c, k, i, S.h_in[i], S.hpw[i], [] {});
+  else
+    cell_upwind<T, NC>(m, S, L, c, k, i);
 }
 
 // Diagnostics of a state (u, h): at cells kdiv = ke - nu div, whose edge
@@ -262,16 +282,15 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
     L.split(i, c, k);
     if constexpr (T > 0) {
       const double hn = h_next[i], hpv = S.h_prev[i];
-      double tp[T], acc0[T];
+      // one pass over the cell's edges: tracer tendency and the next state's diagnostics
+      CellDiag d{st, S, u_next, L, k};
+      double tend[T], tp[T], acc0[T];
+      cell_tracer_tend<T, NC>(m, S, L, c, k, i, tend, d);
 #pragma unroll
       for (int t = 0; t < T; ++t) {
         tp[t] = S.tr_prev[i * T + t];
         acc0[t] = S.stage == 0 ? 0.0 : S.trh_acc[i * T + t];
       }
-      // one pass over the cell's edges: tracer tendency and the next state's diagnostics
-      CellDiag d{st, S, u_next, L, k};
-      double tend[T];
-      cell_tracer_tend<T, NC>(m, S, L, c, k, i, tend, d);
       d.finish(m, c, i);
       const double rh = rcp_nr(hn);
 #pragma unroll

@@ -205,14 +205,17 @@ struct SwState {
 // and on one that does, the partial last wave and the edge / cell boundary
 // inside a block cost less (level-7 sphere, one FCT tracer: 375 us per step with
 // 64, 376 with 128, 395 with 256; level 6: 117 / 119 / 129; 64 x 64 plane: 60 /
-// 60 / 64).  Ocean app: 128 for the edges (level 6, 60 x 3: 628 / 627 / 651 us
+// 60 / 64); but the short edge pre-pass without FCT, which strides over many
+// items, 256 on large meshes (level 7, 3 levels: 43.3 -> 42.0 us per launch; 151 x
+// 98 plane, 5 levels: 14.3 -> 13.0 with 64).  Ocean app: 128 for the edges (level 6, 60 x 3: 628 / 627 / 651 us
 // per launch); the cell kernels 256 where their blocks fill every SM (cells 471 /
 // 467 / 455, final 384 / 382 / 363), else 128 (77 x 54 plane, 7 x 1: 96.7 / 94.5 /
 // 97.9 us per step).
 inline int stage_tpb(const SwState &s, int k) {
   if (!s.tune_auto) return s.tune_tpb[k];
-  if (s.p.app != MPASO_APP_OCEAN) return 64;
   const MeshCtx &c = s.mesh->ctx;
+  if (s.p.app != MPASO_APP_OCEAN)
+    return k == 0 && !s.p.fct && (int64_t)c.d.nE * s.L >= 4096LL * c.sms ? 256 : 64;
   return k == 0 || (int64_t)c.d.nC * s.L < 1024LL * c.sms ? 128 : 256;
 }
 
@@ -337,26 +340,33 @@ __device__ __forceinline__ void for_slots(int n, Body &&body) {
 // v in a real slot, +0 in a pad slot (a select on the integer pipe)
 __device__ __forceinline__ double dmask(double v, bool valid) { return valid ? v : 0.0; }
 
-// Cell bounds, upwind tendency and limiter factors R+ / R- (ocean solve.cc:194-267).
+// Upwind sum of a cell without FCT (the centred flux's, apps/sw/tasks/solve.cc:255-269).
 template <int T, int NC>
+__device__ __forceinline__ void cell_upwind(const DMesh &m, const Stage &S, Lev L, int c, int k, int64_t i) {
+  double tl[T];
+#pragma unroll
+  for (int t = 0; t < T; ++t) tl[t] = 0.0;
+  for_slots<NC>(m.nEoC[c], [&](int j, bool ok) {
+    const int64_t s = (int64_t)j * m.nC + c;
+    const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;
+    const long long sm = sign_mask(m.eocSign[s]);
+#pragma unroll
+    for (int t = 0; t < T; ++t) tl[t] += dmask(dflip(S.LO[ie0 + t], sm), ok);
+  });
+#pragma unroll
+  for (int t = 0; t < T; ++t) S.tLO[i * T + t] = tl[t];  // area-weighted; divided by the area later
+}
+
+// Cell bounds, upwind tendency and limiter factors R+ / R- (ocean solve.cc:194-267).
+// `between()` runs once, behind the loads of the cell's neighbours and edges and
+// ahead of the stores (the sw driver's thickness update, which stores too).
+template <int T, int NC, class Between>
 __device__ __forceinline__ void cell_limiter(const DMesh &m, const Stage &S, Lev L, int c, int k,
-                                             int64_t i, double hin, double hpi) {
+                                             int64_t i, double hin, double hpi, Between &&between) {
   const int n = m.nEoC[c];
   double tl[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) tl[t] = 0.0;
-  if (!S.fct) {
-    for_slots<NC>(n, [&](int j, bool ok) {
-      const int64_t s = (int64_t)j * m.nC + c;
-      const int64_t ie0 = ((int64_t)m.eoc[s] * L + k) * T;
-      const long long sm = sign_mask(m.eocSign[s]);
-#pragma unroll
-      for (int t = 0; t < T; ++t) tl[t] += dmask(dflip(S.LO[ie0 + t], sm), ok);
-    });
-#pragma unroll
-    for (int t = 0; t < T; ++t) S.tLO[i * T + t] = tl[t];  // area-weighted; divided by the area later
-    return;
-  }
   double trc[T], mx[T], mn[T], fi[T], fo[T];
 #pragma unroll
   for (int t = 0; t < T; ++t) {
@@ -386,6 +396,7 @@ __device__ __forceinline__ void cell_limiter(const DMesh &m, const Stage &S, Lev
   const double dtia = S.dt * m.invAreaCell[c];  // dt / area
   const double dthi = dtia * hpi;               // dt / (area hProv)
   const double eps = 1.e-10;
+  between();
 #pragma unroll
   for (int t = 0; t < T; ++t) {
     // trUp = (tr h + dt tend) / hProv; trMaxNew - trUp = dt flxIn / hProv, with
