@@ -28,6 +28,7 @@
 #include <utility>
 
 #include "rk4.cuh"
+#include "softmul.cuh"
 
 namespace mpaso {
 namespace {
@@ -92,6 +93,22 @@ template <int LANES> __device__ __forceinline__ double lane_total(double x) {
   return x;
 }
 
+// K2 is bound by the FP64 pipe (82% busy at level 7, a fifth of the issue slots
+// used), and the two TRiSK sums are half of an edge's FP64 work.  The flux sum
+// s1 runs on the integer pipe instead (FixedSum; its error is below the FMA
+// chain's), unrolled stencils only: level 7 one FCT tracer 45.0 -> 40.6 us per
+// launch, no tracer 36.4 -> 31.7, 151 x 98 plane of 5 levels 21.8 -> 18.5.  With
+// s2 there as well the integer pipe bounds it (41.0, 32.5, 18.5).
+//
+// sum_j W_j/8 F2_j of an edge in hardware arithmetic, where FixedSum does not hold.
+__device__ __noinline__ double trisk_flux_outside(const int *eoe, const double *w, const double2 *FG, int nE, int e,
+                                                  int ne, int L, int k) {
+  double s = 0.0;
+  for (int j = 0; j < ne; ++j)
+    s = fma(w[(int64_t)j * nE + e], FG[(int64_t)eoe[(int64_t)j * nE + e] * L + k].x, s);
+  return s;
+}
+
 template <int T, int NW, int SPLIT, int LANES = 1>
 __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
   const int64_t nEL = (int64_t)m.nE * L;
@@ -101,6 +118,8 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
     const int e = (int)(i / (int)L), k = (int)(i - (int64_t)e * L);
     // q = sum_j W_j F_j (pv_e + pv_j) / 2 = (Pv_e sum W/8 F2_j + sum W/8 F2_j Pv_j)
     double s1 = 0.0, s2 = 0.0;
+    constexpr bool fixed = NW > 0 && LANES == 1;
+    FixedSum sum;
     const int ne = NW > 0 ? NW : m.maxEoE;
 #pragma unroll
     for (int j = lane; j < ne; j += LANES) {
@@ -108,9 +127,14 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
       const double w = __ldcs(st.woe8 + ((int64_t)j * m.nE + e));
       const int64_t io = (int64_t)eo * L + k;
       const double2 fg = S.FG[io];
-      s1 = fma(w, fg.x, s1);
+      if constexpr (fixed)
+        sum.add(fg.x, FixedFactor(w));
+      else
+        s1 = fma(w, fg.x, s1);
       s2 = fma(w, fg.y, s2);
     }
+    if constexpr (fixed)
+      s1 = sum.valid() ? sum.value() : trisk_flux_outside(m.eoe, st.woe8, S.FG, m.nE, e, ne, L, k);
     s1 = lane_total<LANES>(s1);
     s2 = lane_total<LANES>(s2);
     if (lane) return;
@@ -193,8 +217,9 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
   }
 }
 
+// (uncapped, up to one tracer: 64 registers; 40 to 56 were slower: 42.2 us)
 template <int T, int NW, int OC, int SPLIT, int LANES = 1>
-__global__ void MPASO_BOUNDS(OC) k_sw_tend(DMesh m, DStat st, Stage S, Lev L) {
+__global__ void __launch_bounds__(TPB, OC ? 6 : T <= 1 ? 4 : 0) k_sw_tend(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
   tend_item<T, NW, SPLIT, LANES>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }

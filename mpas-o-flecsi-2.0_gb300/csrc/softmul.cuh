@@ -104,6 +104,50 @@ __device__ __forceinline__ double mul_int(double a, double b) {
   return r;
 }
 
+// A sum of up to 15 products on the integer pipe, where it may be rounded as a
+// whole: 64-bit fixed point under the largest exponent so far (the accumulator
+// is shifted down when a term with a larger one comes).  A term is the
+// product's leading 58 bits or more, cut below 2^-57 of the largest term, so the
+// sum's error is below that of a chain of fused multiply-adds, which rounds
+// every partial sum to 53 bits.
+struct FixedFactor {  // one factor of several terms
+  uint32_t h, l, hi;
+  __device__ __forceinline__ explicit FixedFactor(double b) {
+    uint32_t lo;
+    soft_words(b, hi, lo);
+    h = (__funnelshift_l(lo, hi, 10) & 0x3fffffffu) | 0x40000000u, l = lo << 10;
+  }
+};
+struct FixedSum {
+  int64_t acc = 0;
+  uint32_t top = 0;  // largest sum of two biased exponents, in units of 2^20
+  __device__ __forceinline__ void add(double a, const FixedFactor &b) {
+    uint32_t hi, al;
+    soft_words(a, hi, al);
+    const uint32_t x = ((hi & kExp) >> 20) + ((b.hi & kExp) >> 20);
+    const uint32_t ah = (hi & 0xfffffu) | 0x100000u;
+    const uint64_t t0 = (uint64_t)al * b.l;
+    const uint64_t t1 = (uint64_t)ah * b.l + (t0 >> 32);
+    const uint64_t t2 = (uint64_t)al * b.h + t1;
+    const uint64_t t3 = (uint64_t)ah * b.h + (t2 >> 32);
+    // a b 2^10 = t3 2^64 + ..; v = significands' product / 2^47, in [2^57, 2^59)
+    const uint64_t v = ((uint64_t)__funnelshift_l((uint32_t)t3, (uint32_t)(t3 >> 32), 7) << 32) |
+                       __funnelshift_l((uint32_t)t2, (uint32_t)t3, 7);
+    const uint32_t m = max(top, x);
+    const int64_t s = (int32_t)(hi ^ b.hi) >> 31;
+    acc = (acc >> min(m - top, 63u)) + ((int64_t)(v >> min(m - x, 63u)) ^ s) - s;
+    top = m;
+  }
+  // Whether the exponents were such that the sum holds: no infinity or NaN, and
+  // at least one term far enough above the subnormals that zeros and
+  // subnormals (taken as if normal, with exponent 0) were shifted out.
+  __device__ __forceinline__ bool valid() const { return top - 1280u < 1600u; }
+  __device__ __forceinline__ double value() const {
+    const double r = (double)acc;  // rounded to nearest
+    return acc == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (int)((top - 2103u) << 20), __double2loint(r));
+  }
+};
+
 // Rare work of the high-order flux, called so that warps without it skip it: inlined, it becomes
 // predicated instructions, which occupy the FP64 pipe all the same (11 a
 // thread beside the 36 sums of three tracers).
