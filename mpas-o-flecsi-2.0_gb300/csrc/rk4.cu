@@ -247,20 +247,33 @@ __global__ void MPASO_BOUNDS(OC) k_sw_limit(DMesh m, Stage S, Lev L) {
 // into the same cell function would save two more instructions per edge but
 // leaves an absolute error floor of ulp(g h) / dcEdge in tend_u, which breaks
 // the relative parity bar for slow flows.)
-struct CellDiag {
+__device__ __noinline__ double cell_ke_outside(const int *eoc, const double *kw, const double *u, int nC, int c, int n,
+                                               int L, int k) {
+  double ke = 0.0;
+  for (int j = 0; j < n; ++j) {
+    const int e = eoc[(int64_t)j * nC + c];
+    const double ue = u[(int64_t)e * L + k];
+    ke = fma(kw[e], ue * ue, ke);
+  }
+  return ke;
+}
+// SOFT: squares on the integer pipe (Stage::fill).
+template <bool SOFT> struct CellDiag {
   const DStat &st;
   const Stage &S;
   const double *u;
   Lev L;
   int k;
   double ke = 0.0, dv = 0.0;
+  uint32_t bad = 0;
   __device__ void operator()(int64_t s, int e, bool valid) {
     const double ue = u[(int64_t)e * L + k];
-    const double kn = fma(st.kw[e], ue * ue, ke);
+    const double kn = fma(st.kw[e], SOFT ? soft_square(ue, bad) : ue * ue, ke);
     ke = valid ? kn : ke;
     if (S.visc) dv = fma(st.sdv[s], ue, dv);  // sdv is 0 in pad slots
   }
-  __device__ void finish(const DMesh &m, int c, int64_t i) const {
+  __device__ void finish(const DMesh &m, int c, int64_t i) {
+    if (SOFT && bad) ke = cell_ke_outside(m.eoc, st.kw, u, m.nC, c, m.nEoC[c], L, k);
     double b = ke * m.invAreaCell[c];
     // sdv = edgeSignOnCell dv is inward-positive: div = -dv / area, -nu div = nu dv / area
     if (S.visc) b = fma(st.nuInva[c], dv, b);
@@ -268,10 +281,10 @@ struct CellDiag {
   }
 };
 
-template <int NC>
+template <int NC, bool SOFT>
 __device__ __forceinline__ void cell_diag(const DMesh &m, const DStat &st, const Stage &S, Lev L,
                                           int c, int k, int64_t i, const double *u) {
-  CellDiag d{st, S, u, L, k};
+  CellDiag<SOFT> d{st, S, u, L, k};
   for_slots<NC>(m.nEoC[c], [&](int j, bool ok) {
     const int64_t s = (int64_t)j * m.nC + c;
     d(s, m.eoc[s], ok);
@@ -289,9 +302,17 @@ __device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, con
     circ = fma(st.sdc[s], u[(int64_t)m.eov[s] * L + k], circ);
     hs = fma(m.kite[s], h[(int64_t)m.cov[s] * L + k], hs);
   }
-  S.vort[i] = circ * m.invAreaTriangle[v];
   // (f + circ/A) / (hs/A) = (f A + circ) / hs
-  const double pv = fma(m.fVertex[v], m.areaTriangle[v], circ) * rcp_nr(hs);
+  const double ia = m.invAreaTriangle[v], num = fma(m.fVertex[v], m.areaTriangle[v], circ), rh = rcp_nr(hs);
+  double vort, pv;
+  if (S.fill) {
+    uint32_t bad = 0;
+    vort = soft_mul(circ, soft_factor(ia, bad), bad), pv = soft_mul(num, soft_factor(rh, bad), bad);
+    if (bad) vort = product_outside(circ, ia), pv = product_outside(num, rh);
+  } else {
+    vort = circ * ia, pv = num * rh;
+  }
+  S.vort[i] = vort;
   S.pv[i] = pv;
   if (S.tape_pv) S.tape_pv[i] = pv, S.tape_hs[i] = hs;
 }
@@ -308,7 +329,7 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
     if constexpr (T > 0) {
       const double hn = h_next[i], hpv = S.h_prev[i];
       // one pass over the cell's edges: tracer tendency and the next state's diagnostics
-      CellDiag d{st, S, u_next, L, k};
+      CellDiag<false> d{st, S, u_next, L, k};
       double tend[T], tp[T], acc0[T];
       cell_tracer_tend<T, NC>(m, S, L, c, k, i, tend, d);
 #pragma unroll
@@ -331,7 +352,10 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
         }
       }
     } else {
-      cell_diag<NC>(m, st, S, L, c, k, i, u_next);
+      if (S.fill)
+        cell_diag<NC, true>(m, st, S, L, c, k, i, u_next);
+      else
+        cell_diag<NC, false>(m, st, S, L, c, k, i, u_next);
     }
     return;
   }
@@ -357,7 +381,7 @@ __global__ void __launch_bounds__(TPB) k_sw_diag(DMesh m, DStat st, Stage S, Lev
   if (i < nCL) {
     int c, k;
     L.split(i, c, k);
-    cell_diag<NC>(m, st, S, L, c, k, i, S.u_in);
+    cell_diag<NC, false>(m, st, S, L, c, k, i, S.u_in);
     return;
   }
   i -= nCL;
@@ -548,6 +572,7 @@ Stage make_stage(SwState &s, int rk, double dt) {
   const double rk_sub[4] = {dt / 2, dt / 2, dt, 0};
   Stage S{};
   S.stage = rk, S.w_sub = rk_sub[rk], S.w_acc = rk_w[rk], S.dt = dt, S.g = s.p.gravity, S.nu = s.p.nu;
+  S.fill = fills_gpu(s);
   S.fct = s.p.fct, S.hmix = s.p.hmix, S.visc = s.p.nu != 0.0, S.pin_u = s.p.pin_u, S.centred = !s.p.fct;
   // buffer rotation: prev = 0, acc = 2, stage inputs 0 -> 1 -> 3 -> 1, new -> 0
   static const int uin[4] = {0, 1, 3, 1}, uout[4] = {1, 3, 1, -1};

@@ -95,6 +95,12 @@ struct Stage {
   double w_sub, w_acc;  // substep and accumulation weights (apps/sw/run.cc:23-24)
   double dt, g, nu;
   int fct, hmix, visc, pin_u;
+  // sw: the mesh fills the GPU, where the last kernel is bound by the FP64 pipe: the
+  // products of the vertex part and (without tracers) the squared velocities go
+  // to the integer pipe, the same values bit for bit, at some hundred cycles of
+  // latency that a smaller mesh would only wait for (level 7, no tracer: 206 -> 197
+  // us per step, one tracer 354 -> 351; level 3 90 -> 92, so not there)
+  int fill;
   int centred;          // without FCT: the sw app's centred tracer flux (1) or no advection (0, ocean)
   const double *u_in, *h_in, *tr_in;        // stage input
   const double *u_prev, *h_prev, *tr_prev;  // step start
@@ -219,6 +225,12 @@ inline int stage_tpb(const SwState &s, int k) {
   return k == 0 || (int64_t)c.d.nC * s.L < 1024LL * c.sms ? 128 : 256;
 }
 
+// Whether the mesh keeps every SM busy (more than 256 edge-levels each).
+inline bool fills_gpu(const SwState &s) {
+  const MeshCtx &c = s.mesh->ctx;
+  return (int64_t)c.d.nE * s.L > 256LL * c.sms;
+}
+
 // Whether consecutive stage kernels of the sw app overlap their launches.
 // Untuned: where a kernel's threads leave most of every SM free (at most 256
 // edge-levels an SM), so that the next kernel's blocks can wait resident beside
@@ -226,8 +238,7 @@ inline int stage_tpb(const SwState &s, int k) {
 // 70.1 -> 66.0; above, the waiting blocks spread unevenly: 24,000 cells 86.7
 // -> 102.6, level 6 117 -> 138.
 inline bool stage_pdl(const SwState &s) {
-  const MeshCtx &c = s.mesh->ctx;
-  return s.tune_auto ? (int64_t)c.d.nE * s.L <= 256LL * c.sms : s.tune_pdl != 0;
+  return s.tune_auto ? !fills_gpu(s) : s.tune_pdl != 0;
 }
 
 // Allocates the state buffers listed as (pointer, doubles) in one arena.

@@ -43,3 +43,33 @@ def test_unrolled_step_equals_runtime_loops(spec, exp2, nlev):
         assert np.array_equal(u1, u0) and not u1.any()
     else:
         assert np.abs(u1 - u0).max() <= 1e-13 * np.abs(u0).max() + 2.0 ** -1070
+
+
+@pytest.mark.parametrize("ntr", [0, 1])
+@pytest.mark.parametrize("exp2", [None, -960, -700, -512, -505, 0])
+def test_gpu_filling_column_equals_its_levels(exp2, ntr):
+    """A mesh that fills the GPU forms some products on the integer pipe that a
+    smaller one leaves to the hardware, bit for bit the same: two levels of a
+    level-5 sphere (61,440 edge-levels, above the line) against each level alone
+    (30,720, below it)."""
+    import mpaso.gpu as G
+    mesh = mpaso.Mesh.icosa(5)
+    h, u, tr = sw_state(mesh, 5, 2, 1)
+    u = np.zeros_like(u) if exp2 is None else np.ldexp(u, exp2)
+    u[::11] = 0.0
+    dm = G.DeviceMesh(mesh)
+
+    def run(lev):
+        st = G.State(dm, nlev=h[:, lev].shape[1], ntr=ntr, hmix=ntr > 0, kappa=1e4, nu=1e4)
+        fields = [(G.FIELD_H, h), (G.FIELD_U, u)] + ([(G.FIELD_TRACERS, tr)] if ntr else [])
+        for f, a in fields:
+            st.set(f, np.ascontiguousarray(a[:, lev]))
+        st.step(100.0, 2)
+        out = [st.get(f) for f, _ in fields] + [st.get(G.FIELD_VORTICITY), st.get(G.FIELD_PV_VERTEX)]
+        st.close()
+        return out
+
+    both = run(slice(0, 2))
+    for k in range(2):
+        for a, b in zip(both, run(slice(k, k + 1))):
+            assert np.array_equal(a[:, k:k + 1], b)
