@@ -334,14 +334,16 @@ __device__ __forceinline__ double combine(int rk, double dt, int64_t i, double m
 
 // B3 (cells + edges): thickness through kites; u through circulation, KE and
 // divergence; then the RK combination.
+// NC = 6: the slots unrolled (pads have a zero kite), so that their gathers overlap.
+template <int NC>
 __device__ __forceinline__ void b3_cell_item(const DMesh &m, const AdjArgs &a, Lev L, int64_t i) {
   int c, k;
   L.split(i, c, k);
   double mh = a.mu_h[i];
-  for (int j = 0; j < m.maxEoC; ++j) {
+  for_slots<NC>(m.maxEoC, [&](int j, bool) {
     const int64_t s = (int64_t)j * m.nC + c;
     mh = fma(m.kiteR[s], a.lhs[(int64_t)m.vocR[s] * L + k], mh);
-  }
+  });
   combine(a.rk, a.dt, i, mh, a.lam_h, a.acc_h, a.lk_h);
 }
 
@@ -361,12 +363,13 @@ __device__ __forceinline__ void b3_edge_item(const DMesh &m, const DStat &st, co
   if (a.prep) prep_edge(m, a, L, e, k, i, a.un, a.hn, a.pvn, lk);
 }
 
+template <int NC>
 __global__ void __launch_bounds__(TPB) k_adj_b3(DMesh m, DStat st, AdjArgs a, Lev L) {
   stage_prologue();
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (i < nCL) {
-    b3_cell_item(m, a, L, i);
+    b3_cell_item<NC>(m, a, L, i);
     return;
   }
   i -= nCL;
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__(TPB) k_adj_b3_tra(DMesh m, DStat st, AdjArgs a
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (i < nCL) {
-    b3_cell_item(m, a, L, i);
+    b3_cell_item<NC>(m, a, L, i);
     tr_a_item<1, NC, false>(m, tn, L, i);
     return;
   }
@@ -690,7 +693,7 @@ __device__ __forceinline__ double add_bounds(double lt, int2 am, const double2 *
 // of q runs (g = lk_q / areaCell for the next stage beside it).  NL lanes per
 // cell split the gathers and sum by shuffles.
 // Returns true on the lane that holds the cell's thickness cotangent mh_out.
-template <int NL>
+template <int NL, int NC>
 __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L, int64_t g, double &mh_out) {
   const int lane = (int)(g & (NL - 1));
   const int64_t i = g / NL;
@@ -702,17 +705,24 @@ __device__ __forceinline__ bool tr_c_item(const DMesh &m, const TrArgs &a, Lev L
   for (int t = 0; t < T; ++t) {
     const int64_t it = i * T + t;
     double lt = 0.0;
-    for (int j = lane; j < n; j += NL) {
+    auto slot = [&](int j, bool ok) {
       const int64_t s = (int64_t)j * m.nC + c;
-      const double2 p = a.p12[((int64_t)m.eoc[s] * L + k) * T + t];
-      lt += (m.nbr[s] & 1) ? p.x : p.y;
+      const int64_t ie = ((int64_t)m.eoc[s] * L + k) * T + t;
+      lt += dmask(reinterpret_cast<const double *>(a.p12 + ie)[(m.nbr[s] & 1) ^ 1], ok);
       if (a.fct) {
-        const int oc = m.cocU[s];
+        const int oc = m.cocU[s];  // -1 in pads
         if (oc >= 0) {
           const int64_t ot = ((int64_t)oc * L + k) * T + t;
           lt = add_bounds(lt, a.amm[ot], a.lmm, ot, c);
         }
       }
+    };
+    if constexpr (NC > 0) {  // unrolled, so that the slots' gathers overlap
+#pragma unroll
+      for (int j = 0; j < NC; j += NL)
+        if (j + NL <= NC || lane < NC - j) slot(j + lane, j + lane < n);
+    } else {
+      for (int j = lane; j < n; j += NL) slot(j, true);
     }
     if (a.fct)
       for (int j0 = lane; j0 < m.maxAdvR; j0 += 4 * NL) {
@@ -831,13 +841,13 @@ __global__ void __launch_bounds__(TPB) k_adj_trb_b1(DMesh m, TrArgs t, AdjArgs a
 // ... and TC and B2: the NL lanes of a cell-level do TC, its first lane then
 // the cell part of B2 with the thickness cotangent in hand; the threads past
 // the cells do B2's vertices.
-template <int NL>
+template <int NL, int NC>
 __global__ void __launch_bounds__(TPB) k_adj_trc_b2(DMesh m, TrArgs t, AdjArgs a, Lev L) {
   int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nCL = (int64_t)m.nC * L;
   if (g < nCL * NL) {
     double mh;
-    if (tr_c_item<NL>(m, t, L, g, mh)) b2_cell_item(m, a, L, g / NL, mh);
+    if (tr_c_item<NL, NC>(m, t, L, g, mh)) b2_cell_item(m, a, L, g / NL, mh);
     return;
   }
   g -= nCL * NL;
@@ -1008,36 +1018,38 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
   if (first && !ocean) launch_pdl(k_adj_prep, nE, TPL, pdl, st, m, a, L);
   if (A.tr) {
     const TrArgs t = tr_args(s, A, rk, j);
-    constexpr int NLA = 1, NLC = 2;  // lanes per cell (measured best at level 6)
+    constexpr int NLA = 1;  // lanes per cell of TA (measured best at level 6)
     if (t.fct && !tra_done) {
       const bool c6 = m.maxEoC <= 6;
       launch_pdl(ocean ? (c6 ? k_adj_tr_a<NLA, 6, true> : k_adj_tr_a<NLA, 0, true>)
                        : (c6 ? k_adj_tr_a<NLA, 6, false> : k_adj_tr_a<NLA, 0, false>),
                  nC * NLA, TPL, pdl, st, m, t, L);
     }
-    // two lanes per cell-level hide gather latency on small meshes; with a
-    // million cell-levels or more there is parallelism enough, and the
-    // second lane only idles through the per-cell tail on the FP64 pipe
-    const bool one_lane = nC >= (1 << 20);
+    // lanes per cell-level of TC: four or two hide gather latency on small meshes
+    // (level 5, one tracer, 24 stages: 4 lanes 1320 us, 2 lanes 1339, 8 lanes 1370);
+    // with a million cell-levels or more there is parallelism enough, and the
+    // other lanes only idle through the per-cell tail on the FP64 pipe
+    const int lanes = nC >= (1 << 20) ? 1 : nC > 256LL * s.mesh->ctx.sms ? 2 : 4;
     if (!ocean) {
       // sw: TB with B1 and TC with B2 as two fused launches, then B3
       if (m.maxEoE == 10)
         launch_pdl(k_adj_trb_b1<10>, nE, TPL, pdl, st, m, t, a, L);
       else
         launch_pdl(k_adj_trb_b1<0>, nE, TPL, pdl, st, m, t, a, L);
-      if (one_lane)
-        launch_pdl(k_adj_trc_b2<1>, nC + nV, TPL, pdl, st, m, t, a, L);
-      else
-        launch_pdl(k_adj_trc_b2<NLC>, nC * NLC + nV, TPL, pdl, st, m, t, a, L);
+      const bool c6 = m.maxEoC == 6;
+      launch_pdl(lanes == 1   ? (c6 ? k_adj_trc_b2<1, 6> : k_adj_trc_b2<1, 0>)
+                 : lanes == 2 ? (c6 ? k_adj_trc_b2<2, 6> : k_adj_trc_b2<2, 0>)
+                              : (c6 ? k_adj_trc_b2<4, 6> : k_adj_trc_b2<4, 0>),
+                 nC * lanes + nV, TPL, pdl, st, m, t, a, L);
       if (t.fct && prep_next) {  // with TA of the next reversed stage (slot j - 1)
         const TrArgs tn = tr_args(s, A, rk > 0 ? rk - 1 : 3, j - 1);
-        if (m.maxEoC <= 6)
+        if (m.maxEoC == 6)
           launch_pdl(k_adj_b3_tra<6>, nC + nE, TPL, pdl, st, m, s.st, a, tn, L);
         else
           launch_pdl(k_adj_b3_tra<0>, nC + nE, TPL, pdl, st, m, s.st, a, tn, L);
         return true;
       }
-      launch_pdl(k_adj_b3, nC + nE, TPL, pdl, st, m, s.st, a, L);
+      launch_pdl(m.maxEoC == 6 ? k_adj_b3<6> : k_adj_b3<0>, nC + nE, TPL, pdl, st, m, s.st, a, L);
       return false;
     }
     launch_pdl(k_adj_oc_tr_b, nE, TPL, pdl, st, m, t, L);
@@ -1051,7 +1063,7 @@ bool stage_vjp(SwState &s, AdjBuffers &A, int rk, int j, bool first, bool prep_n
   else
     launch_pdl(k_adj_b1<0>, nE, TPL, pdl, st, m, a, L);
   launch_pdl(k_adj_b2, nC + nV, TPL, pdl, st, m, a, L);
-  launch_pdl(k_adj_b3, nC + nE, TPL, pdl, st, m, s.st, a, L);
+  launch_pdl(m.maxEoC == 6 ? k_adj_b3<6> : k_adj_b3<0>, nC + nE, TPL, pdl, st, m, s.st, a, L);
   return false;
 }
 

@@ -292,29 +292,38 @@ __device__ __forceinline__ void cell_diag(const DMesh &m, const DStat &st, const
   d.finish(m, c, i);
 }
 
+// Circulation and kite-summed thickness of a vertex: pv = (f A + circ) / hs = num rh.
+struct VertexSums {
+  double circ = 0.0, hs = 0.0, num, rh;
+  __device__ __forceinline__ VertexSums(const DMesh &m, const DStat &st, Lev L, int v, int k, const double *u,
+                                        const double *h) {
+#pragma unroll
+    for (int j = 0; j < kVertexDegree; ++j) {
+      const int64_t s = (int64_t)j * m.nV + v;
+      circ = fma(st.sdc[s], u[(int64_t)m.eov[s] * L + k], circ);
+      hs = fma(m.kite[s], h[(int64_t)m.cov[s] * L + k], hs);
+    }
+    num = fma(m.fVertex[v], m.areaTriangle[v], circ);
+    rh = rcp_nr(hs);
+  }
+};
+
 __device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, const Stage &S, Lev L,
                                             int v, int k, int64_t i, const double *u,
                                             const double *h) {
-  double circ = 0.0, hs = 0.0;
-#pragma unroll
-  for (int j = 0; j < kVertexDegree; ++j) {
-    const int64_t s = (int64_t)j * m.nV + v;
-    circ = fma(st.sdc[s], u[(int64_t)m.eov[s] * L + k], circ);
-    hs = fma(m.kite[s], h[(int64_t)m.cov[s] * L + k], hs);
-  }
-  // (f + circ/A) / (hs/A) = (f A + circ) / hs
-  const double ia = m.invAreaTriangle[v], num = fma(m.fVertex[v], m.areaTriangle[v], circ), rh = rcp_nr(hs);
+  const VertexSums x(m, st, L, v, k, u, h);
+  const double ia = m.invAreaTriangle[v];
   double vort, pv;
   if (S.fill) {
     uint32_t bad = 0;
-    vort = soft_mul(circ, soft_factor(ia, bad), bad), pv = soft_mul(num, soft_factor(rh, bad), bad);
-    if (bad) vort = product_outside(circ, ia), pv = product_outside(num, rh);
+    vort = soft_mul(x.circ, soft_factor(ia, bad), bad), pv = soft_mul(x.num, soft_factor(x.rh, bad), bad);
+    if (bad) vort = product_outside(x.circ, ia), pv = product_outside(x.num, x.rh);
   } else {
-    vort = circ * ia, pv = num * rh;
+    vort = x.circ * ia, pv = x.num * x.rh;
   }
   S.vort[i] = vort;
   S.pv[i] = pv;
-  if (S.tape_pv) S.tape_pv[i] = pv, S.tape_hs[i] = hs;
+  if (S.tape_pv) S.tape_pv[i] = pv, S.tape_hs[i] = x.hs;
 }
 
 // ------------------------------------------------------ K3: cells + vertices
@@ -370,6 +379,32 @@ template <int T, int NC, int OC>
 __global__ void MPASO_BOUNDS(OC) k_sw_final(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
   final_item<T, NC>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+}
+
+// K3 and the next stage's K1 in one launch, for stages without tracers on meshes
+// that do not fill the GPU, where a launch and its chain of round trips cost
+// more than work done twice: an edge forms the pv of its two vertices itself
+// (as vertex_diag does, each product rounded on its own) instead of waiting
+// for the vertices' threads.  Nine launches a step instead of twelve: level 3
+// 35.3 -> 31.2 us, level 4 37.4 -> 31.2, 64 x 64 plane 35.2 -> 31.2, level 5 39.4.
+template <int NC>
+__global__ void __launch_bounds__(TPB) k_sw_final_pre(DMesh m, DStat st, Stage S, Lev L) {
+  stage_prologue();
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t nEL = (int64_t)m.nE * L;
+  if (i >= nEL) {
+    final_item<0, NC>(m, st, S, L, i - nEL);
+    return;
+  }
+  int e, k;
+  L.split(i, e, k);
+  const int2 c = m.coe[e], v = m.voe[e];
+  const double hs = S.h_out[(int64_t)c.x * L + k] + S.h_out[(int64_t)c.y * L + k];  // 2 h_edge
+  const double F = S.u_out[i] * hs;                                                 // 2 u h_edge
+  const VertexSums a(m, st, L, v.x, k, S.u_out, S.h_out), b(m, st, L, v.y, k, S.u_out, S.h_out);
+  const double pv2 = __dmul_rn(a.num, a.rh) + __dmul_rn(b.num, b.rh);               // 2 pv_edge
+  S.FG[i] = make_double2(F, F * pv2);
+  S.pve[i] = pv2;
 }
 
 // Initial diagnostics (apps/sw/run.cc:88-92).
@@ -683,12 +718,15 @@ void launch_k3(const SwState &s, const Stage &S, bool unroll, int b, cudaStream_
 template <int T> void launch_stage_T(SwState &s, const Stage &S, cudaStream_t st) {
   const DMesh &m = s.mesh->ctx.d;
   cudaEvent_t *ev = s.prof_events;
+  // the first stage of a step runs K1, the others found its work done
+  const bool fused = T == 0 && stage_fused(s);
   // 10-slot edge stencils (K1, K2 edges) and at most 6 edges per cell (K2, K3 cells)
   const bool w10 = m.maxEoE == 10 && (m.maxAdv == 10 || !s.p.fct || T == 0), c6 = m.maxEoC <= 6;
   constexpr int OC1 = T <= kOccMaxT ? 1 : 0;  // no capped variants compiled beyond kOccMaxT
   const bool split = T > 0 && s.tune_split;    // four-launch schedule
   const bool u1 = w10 && s.tune_unroll[0], u2 = w10 && c6 && s.tune_unroll[1];
-  if (split) {  // K1 does the thickness flux part only (the T = 0 kernel)
+  if (fused && S.stage > 0) {
+  } else if (split) {  // K1 does the thickness flux part only (the T = 0 kernel)
     if (s.tune_occ[0])
       launch_k1<0, 1>(s, S, u1, stage_tpb(s, 0), st);
     else
@@ -711,7 +749,10 @@ template <int T> void launch_stage_T(SwState &s, const Stage &S, cudaStream_t st
   }
   if (ev) prof_mark(ev[1], st);
   if (s.k2_mark) MPASO_CUDA(cudaEventRecord(s.k2_mark, st));
-  if (OC1 && s.tune_occ[2])
+  if (fused && S.stage < 3)
+    launch_ex(c6 ? k_sw_final_pre<6> : k_sw_final_pre<0>, ((int64_t)m.nE + m.nC + m.nV) * s.L, stage_tpb(s, 2), false, s,
+              st, m, s.st, S, s.L);
+  else if (OC1 && s.tune_occ[2])
     launch_k3<T, OC1>(s, S, c6 && s.tune_unroll[2], stage_tpb(s, 2), st);
   else
     launch_k3<T, 0>(s, S, c6 && s.tune_unroll[2], stage_tpb(s, 2), st);
@@ -1575,7 +1616,7 @@ int mpaso_state_stream(mpaso_state s, void **stream) {
 int mpaso_state_launches_per_step(mpaso_state s, int32_t *n) {
   return guarded("mpaso_state_launches_per_step", [&] {
     require(s && n, MPASO_ERR_ARG, "null argument");
-    *n = s->s.p.app == MPASO_APP_OCEAN ? ocean_launches_per_step(s->s) : 12;
+    *n = s->s.p.app == MPASO_APP_OCEAN ? ocean_launches_per_step(s->s) : s->s.T == 0 && stage_fused(s->s) ? 9 : 12;
   });
 }
 

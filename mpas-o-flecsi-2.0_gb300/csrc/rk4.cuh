@@ -241,6 +241,10 @@ inline bool stage_pdl(const SwState &s) {
   return s.tune_auto ? !fills_gpu(s) : s.tune_pdl != 0;
 }
 
+// Whether stages without tracers run K3 with the next stage's K1 (k_sw_final_pre);
+// not while the kernels are timed one by one.
+inline bool stage_fused(const SwState &s) { return s.tune_auto && !s.prof_events && !fills_gpu(s); }
+
 // Allocates the state buffers listed as (pointer, doubles) in one arena.
 void alloc_arena(SwState &s, std::vector<std::pair<double **, int64_t>> &bufs);
 void build_stat(SwState &s);

@@ -73,3 +73,29 @@ def test_gpu_filling_column_equals_its_levels(exp2, ntr):
     for k in range(2):
         for a, b in zip(both, run(slice(k, k + 1))):
             assert np.array_equal(a[:, k:k + 1], b)
+
+
+@pytest.mark.parametrize("spec", [("icosa", 2), ("icosa", 4), ("hex", 12, 10)])
+@pytest.mark.parametrize("nlev", [1, 3])
+def test_fused_launches_equal_separate_ones(spec, nlev):
+    """Without tracers a small mesh runs the last kernel of a stage with the first
+    of the next; a set launch configuration (here the default's block size) runs
+    them one by one: bit for bit the same fields and diagnostics."""
+    import mpaso.gpu as G
+    mesh = mpaso.Mesh.icosa(spec[1]) if spec[0] == "icosa" else mpaso.Mesh.hex(spec[1], spec[2], 20e3, 1e-4)
+    h, u, _ = sw_state(mesh, 9, nlev, 0)
+    dm = G.DeviceMesh(mesh)
+    got = []
+    for configured in (False, True):
+        st = G.State(dm, nlev=nlev, ntr=0, nu=1e4)
+        if configured:
+            st.set_launch_config([1] * 3, [64] * 3)
+        assert st.launches_per_step() == (12 if configured else 9)
+        st.set(G.FIELD_H, h)
+        st.set(G.FIELD_U, u)
+        st.step(50.0, 2)
+        st.step_graph(50.0, 2)
+        got.append([st.get(f) for f in (G.FIELD_H, G.FIELD_U, G.FIELD_VORTICITY, G.FIELD_PV_VERTEX)])
+        st.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
