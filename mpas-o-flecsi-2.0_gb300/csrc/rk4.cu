@@ -327,7 +327,9 @@ __device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, con
 }
 
 // ------------------------------------------------------ K3: cells + vertices
-template <int T, int NC>
+// SOFT: the cells' squares and tracer products on the integer pipe, bit for bit the
+// same (launch_k3 says when).
+template <int T, int NC, bool SOFT = false>
 __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
   const int64_t nCL = (int64_t)m.nC * L;
   const double *u_next = S.stage == 3 ? S.u_new : S.u_out;
@@ -338,7 +340,7 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
     if constexpr (T > 0) {
       const double hn = h_next[i], hpv = S.h_prev[i];
       // one pass over the cell's edges: tracer tendency and the next state's diagnostics
-      CellDiag<false> d{st, S, u_next, L, k};
+      CellDiag<SOFT> d{st, S, u_next, L, k};
       double tend[T], tp[T], acc0[T];
       cell_tracer_tend<T, NC>(m, S, L, c, k, i, tend, d);
 #pragma unroll
@@ -348,16 +350,32 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
       }
       d.finish(m, c, i);
       const double rh = rcp_nr(hn);
+      // thickness-weighted tracer RK (apps/sw/tasks/solve.cc:162, 300-302, 337, 354)
+      double tr[T], acc[T];
+      auto update = [&](auto &&times_h, auto &&over_h) {
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+          const double hp_tp = times_h(tp[t]);
+          acc[t] = fma(S.w_acc, tend[t], S.stage == 0 ? hp_tp : acc0[t]);
+          tr[t] = over_h(S.stage == 3 ? acc[t] : fma(S.w_sub, tend[t], hp_tp));
+        }
+      };
+      if constexpr (SOFT) {
+        uint32_t bad = 0;
+        const SoftFactor fh = soft_factor(hpv, bad), fr = soft_factor(rh, bad);
+        update([&](double x) { return soft_mul(x, fh, bad); }, [&](double x) { return soft_mul(x, fr, bad); });
+        if (bad)
+          update([&](double x) { return product_outside(x, hpv); }, [&](double x) { return product_outside(x, rh); });
+      } else {
+        update([&](double x) { return hpv * x; }, [&](double x) { return x * rh; });
+      }
 #pragma unroll
       for (int t = 0; t < T; ++t) {
-        // thickness-weighted tracer RK (apps/sw/tasks/solve.cc:162, 300-302, 337, 354)
-        const double hp_tp = hpv * tp[t];
-        const double acc = fma(S.w_acc, tend[t], S.stage == 0 ? hp_tp : acc0[t]);
         if (S.stage == 3) {
-          S.tr_new[i * T + t] = acc * rh;
+          S.tr_new[i * T + t] = tr[t];
         } else {
-          S.tr_out[i * T + t] = fma(S.w_sub, tend[t], hp_tp) * rh;
-          S.trh_acc[i * T + t] = acc;
+          S.tr_out[i * T + t] = tr[t];
+          S.trh_acc[i * T + t] = acc[t];
         }
       }
     } else {
@@ -375,10 +393,10 @@ __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, cons
   vertex_diag(m, st, S, L, v, k, i, u_next, h_next);
 }
 
-template <int T, int NC, int OC>
+template <int T, int NC, int OC, bool SOFT = false>
 __global__ void MPASO_BOUNDS(OC) k_sw_final(DMesh m, DStat st, Stage S, Lev L) {
   stage_prologue();
-  final_item<T, NC>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
+  final_item<T, NC, SOFT>(m, st, S, L, blockIdx.x * (int64_t)blockDim.x + threadIdx.x);
 }
 
 // K3 and the next stage's K1 in one launch, for stages without tracers on meshes
@@ -709,6 +727,14 @@ template <int T, int OC>
 void launch_k3(const SwState &s, const Stage &S, bool unroll, int b, cudaStream_t st) {
   const DMesh &m = s.mesh->ctx.d;
   const int64_t n = ((int64_t)m.nC + m.nV) * s.L;
+  // The cells' products on the integer pipe: with several levels, whose threads
+  // share the mesh's arrays, the kernel is bound by the FP64 pipe (level 6, 5
+  // levels, no FCT 30.7 -> 28.6 us, 3 FCT tracers 46.7 -> 44.5; level 5, 14 levels, 3
+  // tracers 34.2 -> 30.5); with one level (12.2 -> 14.3) or one FCT tracer (30.7 ->
+  // 30.9) it waits for its gathers, which the test between them holds up
+  if constexpr (T > 0 && !OC)
+    if (unroll && S.fill && s.L > 1 && (T > 1 || !S.fct))
+      return launch_ex(k_sw_final<T, 6, 0, true>, n, b, false, s, st, m, s.st, S, s.L);
   if (unroll)
     launch_ex(k_sw_final<T, 6, OC>, n, b, false, s, st, m, s.st, S, s.L);
   else

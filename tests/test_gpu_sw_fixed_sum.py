@@ -45,7 +45,7 @@ def test_unrolled_step_equals_runtime_loops(spec, exp2, nlev):
         assert np.abs(u1 - u0).max() <= 1e-13 * np.abs(u0).max() + 2.0 ** -1070
 
 
-@pytest.mark.parametrize("ntr", [0, 1])
+@pytest.mark.parametrize("ntr", [0, 1, 2])
 @pytest.mark.parametrize("exp2", [None, -960, -700, -512, -505, 0])
 def test_gpu_filling_column_equals_its_levels(exp2, ntr):
     """A mesh that fills the GPU forms some products on the integer pipe that a
@@ -54,7 +54,8 @@ def test_gpu_filling_column_equals_its_levels(exp2, ntr):
     (30,720, below it)."""
     import mpaso.gpu as G
     mesh = mpaso.Mesh.icosa(5)
-    h, u, tr = sw_state(mesh, 5, 2, 1)
+    h, u, tr = sw_state(mesh, 5, 2, ntr)
+    tr[::13] = 0.0
     u = np.zeros_like(u) if exp2 is None else np.ldexp(u, exp2)
     u[::11] = 0.0
     dm = G.DeviceMesh(mesh)
