@@ -139,7 +139,7 @@ struct SwState {
   void *arena = nullptr;
   size_t arena_bytes = 0;
   double *U[4]{}, *H[4]{}, *TR0 = nullptr, *TRA = nullptr, *TRB = nullptr, *TRH = nullptr;
-  double *HE = nullptr, *HPI = nullptr;
+  double *HE = nullptr, *HPI = nullptr, *SF = nullptr;  // SF: ocean, [maxEoC][nC]
   double *pv = nullptr, *vort = nullptr, *bern = nullptr;
   double *F = nullptr, *pve = nullptr, *A = nullptr, *LO = nullptr, *DF = nullptr;
   double2 *FG = nullptr, *R2 = nullptr;

@@ -78,3 +78,26 @@ def test_ocean_tasks_at_the_window_of_the_integer_products(exp2, ntr):
     S.call("oc_hmix_del2", om, st, cfg, hE, tr, b["tend"], 1e4)
     for k in a:
         assert np.array_equal(a[k], b[k]), k
+
+
+def test_prepared_thickness_on_a_mesh_that_fills_the_gpu():
+    """The thickness flux and 1/hProv in two launches (158,000 cell-levels and more)
+    against the oracle: a level-5 sphere of 16 levels, one step, value for value."""
+    import mpaso.gpu as G
+    mesh = mpaso.Mesh.icosa(5)
+    L, T, dt = 16, 1, 600.0
+    f = fct_statics(mesh, L)
+    h, hE, u, tr = ocean_state(mesh, 6, L, T)
+    rng = np.random.default_rng(9)
+    h, hE = h * rng.uniform(0.9, 1.1, h.shape), hE * rng.uniform(0.9, 1.1, hE.shape)
+    u[rng.uniform(size=u.shape) < 0.1] = 0.0
+    opts = dict(fct=True, hmix=True, kappa=1e4)
+    S = Oracle("restatement")
+    want = S.ocean_run(mesh, S.static(mesh, f), S.config(L, T, **opts), dt, 1, h, hE, u, tr)
+    dm = G.DeviceMesh(mesh, fct=f)
+    st = G.State(dm, app=G.APP_OCEAN, nlev=L, ntr=T, **opts)
+    for field, a in ((G.FIELD_H, h), (G.FIELD_LAYER_THICKNESS_EDGE, hE), (G.FIELD_U, u), (G.FIELD_TRACERS, tr)):
+        st.set(field, a)
+    st.step(dt, 1)
+    got = st.get(G.FIELD_TRACERS)
+    assert np.array_equal(got, np.asarray(want).reshape(got.shape))
