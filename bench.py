@@ -277,8 +277,9 @@ def gpu_arm(args, cfg, extras=True):
             "step_frac": round(step_fp64 / (ms_step * 1e-3) / pipe_peak, 4),
             "instructions_per_cell_update": round(step_fp64 / units_rank, 1),
             "per_kernel_frac": {k: round(model[k][1] / (prof[k] * 1e-3) / pipe_peak, 4) for k in model},
-            "note": "FP64 thread instructions from mpaso/perfmodel.py (within 4% of ncu's counts, tests/test_perfmodel.py) over the "
-                    "graph-replayed time; the FP64 pipe, not HBM, is the binding ceiling of this path"}
+            "note": "FP64 operations of the algorithm from mpaso/perfmodel.py (tests/test_perfmodel.py) over the "
+                    "graph-replayed time, as a share of the FP64 pipe; the ocean kernels' products and the sw TRiSK "
+                    "flux sum run on the integer pipe (csrc/softmul.cuh), so the share may exceed 1"}
     kernels = {k: {"ms_per_launch": round(v, 5), "share": round(v / sum(prof.values()), 3),
                    "model_bytes": int(model[k][0]),
                    "model_gbs": round(model[k][0] / (v * 1e-3) / 1e9, 1),
@@ -906,7 +907,8 @@ def ensemble_arm(args):
                   "ceiling_speedup_vs_serial": (t_serial / K) / (fp64_step / pipe_peak),
                   "note": "FP64 thread instructions of all members' steps (model) over the batch time, against "
                           "2 per clock per SM at 2070 MHz; ceiling = the serial time over the time the batch's "
-                          "FP64 work takes at the pipe's peak"}
+                          "FP64 work takes at the pipe's peak (with all of it on that pipe; the TRiSK flux sum "
+                          "runs on the integer pipe)"}
     out = None
     if rank == 0:
         out = {"metric": "ensemble members*steps/s (one graph-captured launch sequence vs one at a time)",

@@ -7,8 +7,11 @@ again.  FP64 work: DADD / DMUL / DFMA thread instructions per launch (a
 reciprocal by rcp_nr is 4 on the FP64 pipe plus the approximation on the
 special-function unit; the limiter's two guarded quotients run only where a
 bound is active, counted as a quarter of the cells); min/max/select/sign work
-runs on the integer pipe and is not counted.  ncu's counts for the same
-launches are in profiles/ (within about 10% of these).
+runs on the integer pipe and is not counted.  These are the algorithm's
+operations: what the kernels now form on the integer pipe instead (the ocean's
+products, the sw TRiSK flux sum and some products of the last sw kernel,
+csrc/softmul.cuh) is counted as well, so ncu's FP64 counts in profiles/ are
+lower by that.
 
 One cell-update = one cell x one level advanced by one full RK4 step.
 
