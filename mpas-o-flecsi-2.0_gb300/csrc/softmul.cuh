@@ -139,9 +139,11 @@ struct FixedFactor {  // one factor of several terms
 struct FixedSum {
   int64_t acc = 0;
   uint32_t top = 0;  // largest sum of two biased exponents, in units of 2^20
+  uint32_t any = 0;  // nonzero where some a is
   __device__ __forceinline__ void add(double a, const FixedFactor &b) {
     uint32_t hi, al;
     soft_words(a, hi, al);
+    any |= hi << 1 | al;
     const uint32_t x = ((hi & kExp) >> 20) + ((b.hi & kExp) >> 20);
     const uint32_t ah = (hi & 0xfffffu) | 0x100000u;
     const uint64_t t0 = (uint64_t)al * b.l;
