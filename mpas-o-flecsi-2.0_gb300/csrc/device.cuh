@@ -12,6 +12,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -120,6 +121,7 @@ struct MeshCtx {
   // task call; `d` itself where the context keeps the reference's numbering).
   DMesh ref{};
   bool has_ref = false;
+  std::mutex ref_mutex;  // task calls of several threads
   void *ref_arena = nullptr;
   size_t ref_bytes = 0;
   const DMesh &task_view();

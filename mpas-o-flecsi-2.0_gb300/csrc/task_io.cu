@@ -199,7 +199,11 @@ __global__ void k_to_reference(const T *__restrict__ src, T *__restrict__ dst, c
 
 }  // namespace
 
+// Built on a stream of its own with the thread's capture mode relaxed: the
+// call that needs it first may be recorded into a graph, and the view must
+// exist before that graph is launched.
 const DMesh &MeshCtx::task_view() {
+  std::lock_guard<std::mutex> lock(ref_mutex);
   if (has_ref) return ref;
   bool same = true;
   for (const auto &p : perm)
@@ -240,6 +244,17 @@ const DMesh &MeshCtx::task_view() {
   };
   size_t total = 0;
   for (const Item &t : items) total += bytes_of(t);
+  struct Relaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaStream_t stream = nullptr;
+    Relaxed() { MPASO_CUDA(cudaThreadExchangeStreamCaptureMode(&mode)); }
+    ~Relaxed() {
+      if (stream) cudaStreamDestroy(stream);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+  } own;
+  MPASO_CUDA(cudaStreamCreateWithFlags(&own.stream, cudaStreamNonBlocking));
+  const cudaStream_t stream = own.stream;
   void *arena_new = nullptr;
   if (cudaMalloc(&arena_new, total) != cudaSuccess) {
     cudaGetLastError();

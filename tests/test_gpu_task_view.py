@@ -85,3 +85,25 @@ def test_output_sharing_memory_with_an_input():
     check(lib().mpaso_sw_compute_scalar_tend(dm.handle, L, T, _ptr(d[0]), _ptr(d[1]), _ptr(d[2]), _ptr(d[2]), None))
     torch.cuda.synchronize()
     assert np.array_equal(d[2].cpu().numpy(), want)
+
+
+def test_first_task_call_on_a_mesh_recorded_into_a_graph():
+    torch = pytest.importorskip("torch")
+    import mpaso.gpu as G
+    from mpaso._lib import check, lib
+    mesh = mpaso.Mesh.icosa(2)
+    L, T = 2, 2
+    dm = G.DeviceMesh(mesh)
+    rng = np.random.default_rng(7)
+    hE, u = rng.uniform(1, 2, (mesh.nEdges, L)), rng.standard_normal((mesh.nEdges, L))
+    tr = rng.uniform(0, 1, (mesh.nCells, L, T))
+    d = [_dev(torch, a, 0) for a in (hE, u, tr, np.zeros_like(tr))]
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        check(lib().mpaso_sw_compute_scalar_tend(dm.handle, L, T, *[_ptr(x) for x in d],
+                                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    assert not d[3].any()
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(d[3].cpu().numpy(), dm.sw_compute_scalar_tend(L, T, hE, u, tr))
