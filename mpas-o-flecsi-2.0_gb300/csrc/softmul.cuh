@@ -110,7 +110,17 @@ __device__ __forceinline__ double soft_square(double a, uint32_t &bad) {
 // few warps need it, and the compiler turns a plain branch around an inlined
 // multiplication into a predicated one, which occupies the FP64 pipe for the
 // whole warp even where no lane takes it.
-static __device__ __noinline__ double product_outside(double a, double b) { return a * b; }
+// A zero times a finite number, the whole of water at rest, stays off that pipe
+// (level-6 ocean at rest, 60 x 3: 7.74 -> 6.55 ms per step, in motion 5.73).
+static __device__ __noinline__ double product_hw(double a, double b) { return a * b; }
+static __device__ __noinline__ double product_outside(double a, double b) {
+  uint32_t ah, al, bh, bl;
+  soft_words(a, ah, al);
+  soft_words(b, bh, bl);
+  const bool zero = ((ah & 0x7fffffffu) | al) == 0 || ((bh & 0x7fffffffu) | bl) == 0;
+  if (zero && (ah & kExp) != kExp && (bh & kExp) != kExp) return __hiloint2double((int)((ah ^ bh) & 0x80000000u), 0);
+  return product_hw(a, b);
+}
 
 // One product on the integer pipe.
 __device__ __forceinline__ double mul_int(double a, double b) {
