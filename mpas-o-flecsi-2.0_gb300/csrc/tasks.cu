@@ -553,7 +553,8 @@ void check_levels(int L, int T) {
 
 void require_fct(TaskIO &io, int L) {
   require(io.ctx().has_fct, MPASO_ERR_ARG, "mesh context was created without FCT statics");
-  require(io.dm().fctLev == L, MPASO_ERR_ARG, "nlev differs from the FCT statics' level count");
+  // (the context's own mesh: io.dm() is there only from stage() on)
+  require(io.ctx().d.fctLev == L, MPASO_ERR_ARG, "nlev differs from the FCT statics' level count");
 }
 
 cudaStream_t plain_stream(mpaso_mesh m, void *stream) {
