@@ -56,7 +56,8 @@ struct Lev {
 // Device view of a mesh context (all pointers are device memory).
 struct DMesh {
   int nC, nE, nV;
-  int maxEoC, maxEoE, maxAdv, fctLev;
+  int maxEoC;  // rows of the cells' slot arrays: the most edges of a cell, at least six
+  int maxEoE, maxAdv, fctLev;
   // ---- cells ----
   const int *nEoC;            // [nC]
   const int *eoc;             // [maxEoC][nC] edgesOnCell, file order

@@ -135,6 +135,9 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
     maxEoC = std::max(maxEoC, (int)c2e.len(c));
   }
   for (int64_t e = 0; e < nE; ++e) maxEoE = std::max(maxEoE, (int)e2e.len(e));
+  // Rows of the cells' slot arrays: the kernels that unroll six slots read six,
+  // also where no cell has as many edges (the level-0 sphere, twelve pentagons).
+  const int rows = std::max(maxEoC, 6);
 
   // ---- permutation ----
   // reorder: 0 keep the numbering; 1 cells along a Hilbert curve, edges and
@@ -256,10 +259,10 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
   // ---- cells ----
   Arena A;
   DMesh &m = ctx.d;
-  m.nC = (int)nC, m.nE = (int)nE, m.nV = (int)nV, m.maxEoC = maxEoC, m.maxEoE = maxEoE;
-  std::vector<int> nEoC(nC), eoc((size_t)maxEoC * nC), eocAsc((size_t)maxEoC * nC), coc((size_t)maxEoC * nC);
-  std::vector<int> nbr((size_t)maxEoC * nC);
-  std::vector<double> eocSign((size_t)maxEoC * nC, 0.0), eocAscSign((size_t)maxEoC * nC, 0.0);
+  m.nC = (int)nC, m.nE = (int)nE, m.nV = (int)nV, m.maxEoC = rows, m.maxEoE = maxEoE;
+  std::vector<int> nEoC(nC), eoc((size_t)rows * nC), eocAsc((size_t)rows * nC), coc((size_t)rows * nC);
+  std::vector<int> nbr((size_t)rows * nC);
+  std::vector<double> eocSign((size_t)rows * nC, 0.0), eocAscSign((size_t)rows * nC, 0.0);
   std::vector<double> area(nC), invArea(nC), hs(nC, 0.0);
   std::vector<int> mlc(nC, 1);
   const Crs c2eAsc = transpose(e2c, nC);  // edges of each cell, ascending reference id
@@ -267,7 +270,7 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
     const int32_t c = pc[k];
     const int n = (int)c2e.len(c);
     nEoC[k] = n;
-    for (int j = 0; j < maxEoC; ++j) {
+    for (int j = 0; j < rows; ++j) {
       const size_t s = (size_t)j * nC + k;
       if (j < n) {
         const int32_t e = c2e.at(c, j);
@@ -397,8 +400,8 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
       woeT[(size_t)j * nE + k] = woe[(size_t)p * nE + eo];
     }
   });
-  std::vector<int> vocR((size_t)maxEoC * nC, 0);
-  std::vector<double> kiteR((size_t)maxEoC * nC, 0.0);
+  std::vector<int> vocR((size_t)rows * nC, 0);
+  std::vector<double> kiteR((size_t)rows * nC, 0.0);
   std::vector<int> fillc(nC, 0);
   for (int64_t v = 0; v < nV; ++v)
     for (int j = 0; j < kVertexDegree; ++j) {
@@ -409,7 +412,7 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
       fillc[c]++;
     }
   for (int64_t c = 0; c < nC; ++c)
-    for (int j = fillc[c]; j < maxEoC; ++j) vocR[(size_t)j * nC + c] = vocR[c];
+    for (int j = fillc[c]; j < rows; ++j) vocR[(size_t)j * nC + c] = vocR[c];
   A.add(woeT, &m.woeT), A.add(vocR, &m.vocR), A.add(kiteR, &m.kiteR);
   // cell -> entries of the advection stencils that read the cell: the edge
   // (ascending; -1 pads at the end of each column) and the coefficient pair
@@ -460,7 +463,7 @@ void build(MeshCtx &ctx, const mpaso_mesh_desc &d, const std::vector<int64_t> *m
   m.maxAdvR = maxAdvR;
   A.add(advRe, &m.advRe), A.add(advRc, (const double **)&m.advRc);
   // cellsOnCell with the cell itself and repeated neighbours replaced by -1
-  std::vector<int> cocU((size_t)maxEoC * nC, -1);
+  std::vector<int> cocU((size_t)rows * nC, -1);
   parallel_for(nC, [&](int64_t c) {
     for (int j = 0; j < nEoC[c]; ++j) {
       const int o = coc[(size_t)j * nC + c];
