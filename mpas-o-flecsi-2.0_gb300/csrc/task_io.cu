@@ -120,7 +120,7 @@ int64_t TaskIO::count(int entity) const {
 int TaskIO::add(const double *p, int entity, int row, bool output) {
   require(p != nullptr, MPASO_ERR_ARG, "null field pointer");
   require(row >= 1, MPASO_ERR_ARG, "bad row length");
-  Arg a{const_cast<double *>(p), entity, row, output, !is_device_pointer(p), false};
+  Arg a{const_cast<double *>(p), entity, row, output, !is_device_pointer(p)};
   any_host_ |= a.host;
   args_.push_back(a);
   return (int)args_.size() - 1;
@@ -134,7 +134,7 @@ bool TaskIO::overlapping() const {
     const double *x0 = args_[x].user, *x1 = x0 + count(args_[x].entity) * args_[x].row;
     for (size_t y = 0; y < args_.size(); ++y) {
       const double *y0 = args_[y].user, *y1 = y0 + count(args_[y].entity) * args_[y].row;
-      if (x != y && !args_[y].work && x0 < y1 && y0 < x1) return true;
+      if (x != y && x0 < y1 && y0 < x1) return true;
     }
   }
   return false;
@@ -146,16 +146,15 @@ void TaskIO::stage() {
   size_t total = 0;
   auto bytes_of = [&](const Arg &a) { return (size_t)count(a.entity) * a.row * sizeof(double); };
   for (auto &a : args_)
-    if (a.host || a.work || copies_) total += (bytes_of(a) + 255) & ~size_t(255);
+    if (a.host || copies_) total += (bytes_of(a) + 255) & ~size_t(255);
   char *base = total ? (char *)m_->ctx.ensure_scratch(total) : nullptr;
   for (auto &a : args_) {
-    if (!a.host && !a.work && !copies_) {
+    if (!a.host && !copies_) {
       a.internal = a.user;
       continue;
     }
     a.internal = (double *)base;
     base += (bytes_of(a) + 255) & ~size_t(255);
-    if (a.work) continue;
     MPASO_CUDA(cudaMemcpyAsync(a.internal, a.user, bytes_of(a),
                                a.host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, stream_));
   }

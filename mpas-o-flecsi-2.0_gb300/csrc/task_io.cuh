@@ -27,11 +27,6 @@ class TaskIO {
   // keep their values (FleCSI storage semantics): staged outputs are copied in as well.
   int in(const double *p, int entity, int row) { return add(p, entity, row, false); }
   int out(double *p, int entity, int row) { return add(p, entity, row, true); }
-  // A work array of the call's own, uninitialised.
-  int work(int entity, int row) {
-    args_.push_back({nullptr, entity, row, false, false, true});
-    return (int)args_.size() - 1;
-  }
   void stage();                  // copies host arrays in
   double *ptr(int slot) const { return args_[slot].internal; }
   void finish();                 // copies outputs back, syncs for host memory
@@ -43,7 +38,7 @@ class TaskIO {
   struct Arg {
     double *user;
     int entity, row;
-    bool output, host, work = false;
+    bool output, host;
     double *internal = nullptr;
   };
   int add(const double *p, int entity, int row, bool output);

@@ -476,20 +476,27 @@ __global__ void __launch_bounds__(TPB) k_oc_accumulate_fct(DMesh m, Lev L, const
   }
 }
 
-// rho of apps/ocean/tasks/solve.cc:352, once per edge instead of in every
-// cell-level on either side
-__global__ void __launch_bounds__(TPB) k_oc_hmix_rho(DMesh m, double coef, double *rho) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < m.nE) rho[e] = m.meshScalingDel2[e] * coef * m.dvEdge[e] / m.dcEdge[e];
-}
+// apps/ocean/tasks/solve.cc:328-366.  rho (:352) is formed once per cell and slot of
+// the block's cells, in shared memory, instead of in every level.  (An array of
+// the call's own for it, once per edge in a launch ahead, would have to outlive
+// graphs that recorded the call and be private to each stream.)
+constexpr int hmix_cells(int L) { return (L + TPB - 2) / L + 1; }  // most cells that TPB cell-levels touch
 
-// apps/ocean/tasks/solve.cc:328-366
 template <int T>
 __global__ void __launch_bounds__(TPB) k_oc_hmix(DMesh m, Lev L, const double *__restrict__ hE,
-                                                 const double *__restrict__ tr, const double *__restrict__ rho,
-                                                 double *tend) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= (int64_t)m.nC * L) return;
+                                                 const double *__restrict__ tr, double coef, double *tend) {
+  extern __shared__ double rho[];  // [maxEoC][cells of the block]
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x, i = i0 + threadIdx.x, n_all = (int64_t)m.nC * L;
+  int c0, c1, unused;
+  L.split(i0, c0, unused);
+  L.split(min(i0 + blockDim.x, n_all) - 1, c1, unused);
+  const int nc = c1 - c0 + 1;
+  for (int s = threadIdx.x; s < nc * m.maxEoC; s += blockDim.x) {
+    const int j = s / nc, e = m.eoc[(int64_t)j * m.nC + c0 + (s - j * nc)];
+    rho[s] = m.meshScalingDel2[e] * coef * m.dvEdge[e] / m.dcEdge[e];
+  }
+  __syncthreads();
+  if (i >= n_all) return;
   int c, k;
   L.split(i, c, k);
   const double invArea = m.invAreaCell[c];
@@ -504,7 +511,7 @@ __global__ void __launch_bounds__(TPB) k_oc_hmix(DMesh m, Lev L, const double *_
     const int e = m.eoc[s];
     if (k >= m.maxLevelEdgeTop[e]) continue;
     const int2 cc = m.coe[e];
-    const double he = hE[(int64_t)e * L + k], re = rho[e];
+    const double he = hE[(int64_t)e * L + k], re = rho[j * nc + c - c0];
     const EdgeSign sg(m.eocSign[s]);
     uint32_t badm = bada;
     const SoftFactor fh = soft_factor(he, badm), fr = soft_factor(re, badm);
@@ -886,13 +893,12 @@ int mpaso_oc_tracer_hmix_del2_tend(mpaso_mesh m, int32_t nlev, int32_t ntr,
     const int L = nlev, T = ntr;
     const int ihe = io.in(layerThicknessEdge, MPASO_EDGES, L), itr = io.in(tracers, MPASO_CELLS, L * T);
     const int ote = io.out(tend, MPASO_CELLS, L * T);
-    const int rho = io.work(MPASO_EDGES, 1);
     io.stage();
     const DMesh &d = io.dm();
-    k_oc_hmix_rho<<<blocks_for(d.nE, TPB), TPB, 0, io.stream()>>>(d, coef, io.ptr(rho));
+    const size_t shared = (size_t)hmix_cells(L) * d.maxEoC * sizeof(double);  // at most 16 KB
     with_tracers(T, [&](auto t) {
-      k_oc_hmix<t.value><<<blocks_for((int64_t)d.nC * L, TPB), TPB, 0, io.stream()>>>(
-          d, L, io.ptr(ihe), io.ptr(itr), io.ptr(rho), io.ptr(ote));
+      k_oc_hmix<t.value><<<blocks_for((int64_t)d.nC * L, TPB), TPB, shared, io.stream()>>>(
+          d, L, io.ptr(ihe), io.ptr(itr), coef, io.ptr(ote));
     });
     io.finish();
   });
