@@ -48,6 +48,11 @@ struct SoftFactor {
 __device__ __forceinline__ void soft_words(double x, uint32_t &hi, uint32_t &lo) {
   asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
 }
+__device__ __forceinline__ bool nonfinite(double x) {
+  uint32_t hi, lo;
+  soft_words(x, hi, lo);
+  return (hi & kExp) == kExp;
+}
 __device__ __forceinline__ SoftFactor soft_factor(double b, uint32_t &bad) {
   uint32_t hi, lo;
   soft_words(b, hi, lo);

@@ -338,6 +338,19 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_a(DMesh m, Lev L, const double *
   for (int t = 0; t < T; ++t) ho[i * T + t] = x[t] - lo[i * T + t];
 }
 
+// std::min(1, std::max(0, num / den)) (solve.cc:258-265), divided only where the
+// quotient may lie inside (0, 1) or be no number.
+static __device__ __noinline__ double rare_limit(double num, double den) {
+  const double q = num / den, p = (0.0 < q) ? q : 0.0;
+  return (p < 1.0) ? p : 1.0;
+}
+__device__ __forceinline__ double limiter_factor(double num, double den) {
+  const bool pos = dgt0(num);
+  double r = pos ? 1.0 : 0.0;
+  if (!dgt0(den) || nonfinite(num) || nonfinite(den) || (pos && dkey(num) < dkey(den))) r = rare_limit(num, den);
+  return r;
+}
+
 // apps/ocean/tasks/solve.cc:194-214, 232-267: bounds over the cell and its
 // neighbours, per-cell sums and limiter factors.
 template <int T>
@@ -402,8 +415,8 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_b(DMesh m, Lev L, const double *
       const double mnn = up + mul_int(mul_int(fout[t], dt), hpi);
       trMax[it] = mx[t];
       trMin[it] = mn[t];
-      fin[t] = clamp_quotient(mx[t] - up, (mxn - up) + eps);
-      fout[t] = clamp_quotient(up - mn[t], (up - mnn) + eps);
+      fin[t] = limiter_factor(mx[t] - up, (mxn - up) + eps);
+      fout[t] = limiter_factor(up - mn[t], (up - mnn) + eps);
     }
     flxIn[it] = fin[t];
     flxOut[it] = fout[t];
