@@ -312,6 +312,9 @@ __global__ void __launch_bounds__(TPB) k_oc_high_order(DMesh m, Lev L, const dou
   for (int t = 0; t < T; ++t) ho[i * T + t] = flx[t];
 }
 
+// x + tw (t1 + t2) with a weight tw of zero: x unless f or the sum is not finite.
+static __device__ __noinline__ double add_weightless_flux(double x, double f, double sum) { return x + (0.0 * f) * sum; }
+
 // apps/ocean/tasks/solve.cc:216-229: anti-diffusive flux of the edges.  The
 // centred flux has the weight ((mask + 1) & 1), which is 0 on almost all of them.
 template <int T>
@@ -324,18 +327,19 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_a(DMesh m, Lev L, const double *
   L.split(i, e, k);
   if (k >= m.maxLevelEdgeTop[e]) return;
   const bool centred = (m.hoMask[(int64_t)e * m.fctLev + k] + 1) & 1;
-  double x[T];
+  const double f = ntf[i];
+  const int2 c = m.coe[e];
+  const int64_t i1 = ((int64_t)c.x * L + k) * T, i2 = ((int64_t)c.y * L + k) * T;
 #pragma unroll
-  for (int t = 0; t < T; ++t) x[t] = ho[i * T + t];
-  if (centred) {
-    const int2 c = m.coe[e];
-#pragma unroll
-    for (int t = 0; t < T; ++t)
-      x[t] = add_centred_flux(x[t], m.dvEdge[e], ntf[i], tr[((int64_t)c.x * L + k) * T + t],
-                              tr[((int64_t)c.y * L + k) * T + t]);
+  for (int t = 0; t < T; ++t) {
+    double x = ho[i * T + t];
+    const double t1 = tr[i1 + t], t2 = tr[i2 + t], sum = t1 + t2;
+    if (centred)
+      x = add_centred_flux(x, m.dvEdge[e], f, t1, t2);
+    else if (nonfinite(f) || nonfinite(sum))
+      x = add_weightless_flux(x, f, sum);
+    ho[i * T + t] = x - lo[i * T + t];
   }
-#pragma unroll
-  for (int t = 0; t < T; ++t) ho[i * T + t] = x[t] - lo[i * T + t];
 }
 
 // std::min(1, std::max(0, num / den)) (solve.cc:258-265), divided only where the

@@ -45,3 +45,12 @@ def _check(spec, T, arg, value, uneven):
 def test_limiter_factors(spec, T, arg, value):
     """A quotient that is no number counts as 0 (std::max(0, NaN) is 0)."""
     _check(spec, T, arg, value, uneven=False)
+
+
+@pytest.mark.parametrize("value", VALUES)
+@pytest.mark.parametrize("arg", ["ntf", "tr"])
+@pytest.mark.parametrize("spec,T", [(("icosa", 2), 1), (("hex", 9, 6), 3)])
+def test_centred_flux_of_weight_zero(spec, T, arg, value):
+    """Edges with a high-order stencil add the centred flux with a weight of zero,
+    and zero times an infinity or NaN is NaN."""
+    _check(spec, T, arg, value, uneven=False)
