@@ -427,9 +427,18 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_b(DMesh m, Lev L, const double *
   }
 }
 
+// max(0, x) min(in2, out1) + min(0, x) min(out2, in1), both products formed.
+static __device__ __noinline__ double rare_rescale(double x, double in1, double out1, double in2, double out2) {
+  const double a = in2 < out1 ? in2 : out1, b = out2 < in1 ? out2 : in1;
+  return ((0.0 < x) ? x : 0.0) * a + ((x < 0.0) ? x : 0.0) * b;
+}
+
 // apps/ocean/tasks/solve.cc:270-282: rescale anti-diffusive fluxes,
 // max(0, x) min(R-(c1), R+(c2)) + min(0, x) min(R+(c1), R-(c2)), whose factor the
-// sign of x selects.
+// sign of x selects: the other, times zero, counts for nothing where both cells
+// have the level, whose factors k_oc_fct_b put into [0, 1].  In a level below a
+// cell's column (an edge goes down to the deeper of its two cells) flxIn and
+// flxOut are the caller's plus sums, which may be infinite or NaN.
 template <int T>
 __global__ void __launch_bounds__(TPB) k_oc_fct_c(DMesh m, Lev L, const double *__restrict__ flxIn,
                                                   const double *__restrict__ flxOut, double *ho) {
@@ -440,6 +449,11 @@ __global__ void __launch_bounds__(TPB) k_oc_fct_c(DMesh m, Lev L, const double *
   if (k >= m.maxLevelEdgeTop[e]) return;
   const int2 c = m.coe[e];
   const int64_t i1 = ((int64_t)c.x * L + k) * T, i2 = ((int64_t)c.y * L + k) * T;
+  if (k >= m.maxLevelCell[c.x] || k >= m.maxLevelCell[c.y]) {
+    for (int t = 0; t < T; ++t)
+      ho[i * T + t] = rare_rescale(ho[i * T + t], flxIn[i1 + t], flxOut[i1 + t], flxIn[i2 + t], flxOut[i2 + t]);
+    return;
+  }
 #pragma unroll
   for (int t = 0; t < T; ++t) {
     const double x = ho[i * T + t];

@@ -54,3 +54,12 @@ def test_centred_flux_of_weight_zero(spec, T, arg, value):
     """Edges with a high-order stencil add the centred flux with a weight of zero,
     and zero times an infinity or NaN is NaN."""
     _check(spec, T, arg, value, uneven=False)
+
+
+@pytest.mark.parametrize("value", VALUES)
+@pytest.mark.parametrize("arg", ["ho", "lo", "fi", "fo", "tr"])
+@pytest.mark.parametrize("spec,T", [(("icosa", 2), 1), (("hex", 9, 6), 3)])
+def test_levels_below_a_column(spec, T, arg, value):
+    """An edge that goes deeper than one of its cells reads that cell's unlimited
+    flxIn and flxOut, of which the one its flux does not use counts zero times."""
+    _check(spec, T, arg, value, uneven=True)
