@@ -366,10 +366,11 @@ __global__ void __launch_bounds__(TPB, 4) k_oc_final(DMesh m, Stage S, int L) {
         // one product with the minimum the sign selects (integer-pipe selects);
         // a zero flux enters as +0, whose products are the +0 the reference's
         // max(0, A) / min(0, A) terms give
-        // (a zero factor -- local extrema -- makes the flux the zero, the other 1)
+        // (a zero factor -- local extrema -- makes the flux the zero, the other 1,
+        // unless the flux is infinite or NaN, which zero does not make a zero)
         const bool pos = dgt0(a);
         const double rmin = pos ? dmin(r1.y, r2.x) : dmin(r1.x, r2.y);
-        const bool some = dgt0(rmin);
+        const bool some = dgt0(rmin) || nonfinite(a);
         const double a0 = some && (pos || dlt0(a)) ? a : 0.0, r0 = some ? rmin : 1.0;
         td[t] += dflip(soft_mul(soft_mul(a0, soft_factor(r0, bad), bad), fa, bad), sm);
       }
