@@ -138,7 +138,7 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
     }
     if constexpr (fixed)
       s1 = sum.valid() ? sum.value()
-           : sum.any   ? trisk_flux_outside(m.eoe, st.woe8, S.FG, m.nE, e, ne, L, k)
+           : sum.any() ? trisk_flux_outside(m.eoe, st.woe8, S.FG, m.nE, e, ne, L, k)
                        : 0.0;
     s1 = lane_total<LANES>(s1);
     s2 = lane_total<LANES>(s2);

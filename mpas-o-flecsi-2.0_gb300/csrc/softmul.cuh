@@ -154,12 +154,13 @@ struct FixedFactor {  // one factor of several terms
 struct FixedSum {
   int64_t acc = 0;
   uint32_t top = 0;  // largest sum of two biased exponents, in units of 2^20
-  uint32_t any = 0;  // nonzero where some a is
+  uint32_t big = 0, low = 0;  // largest high word of an |a|; its low words' bits together
   __device__ __forceinline__ void add(double a, const FixedFactor &b) {
     uint32_t hi, al;
     soft_words(a, hi, al);
-    any |= hi << 1 | al;
-    const uint32_t x = ((hi & kExp) >> 20) + ((b.hi & kExp) >> 20);
+    const uint32_t mag = hi & 0x7fffffffu;
+    big = max(big, mag), low |= al;
+    const uint32_t x = (mag >> 20) + ((b.hi & kExp) >> 20);
     const uint32_t ah = (hi & 0xfffffu) | 0x100000u;
     const uint64_t t0 = (uint64_t)al * b.l;
     const uint64_t t1 = (uint64_t)ah * b.l + (t0 >> 32);
@@ -173,10 +174,15 @@ struct FixedSum {
     acc = (acc >> min(m - top, 63u)) + ((int64_t)(v >> min(m - x, 63u)) ^ s) - s;
     top = m;
   }
-  // Whether the exponents were such that the sum holds: no infinity or NaN, and
-  // at least one term far enough above the subnormals that zeros and
-  // subnormals (taken as if normal, with exponent 0) were shifted out.
-  __device__ __forceinline__ bool valid() const { return top - 1280u < 1600u; }
+  // Whether some a is not a zero.
+  __device__ __forceinline__ bool any() const { return (big | low) != 0; }
+  // Whether the exponents were such that the sum holds: no a is infinite or NaN,
+  // and the largest term is far above what zeros and subnormals count as, which
+  // is a number of exponent 0 -- as an a beside any b (the first condition), and
+  // as a b beside the largest a.
+  __device__ __forceinline__ bool valid() const {
+    return top - 1280u < 1600u && big < kExp && (big >> 20) + 58u <= top;
+  }
   __device__ __forceinline__ double value() const {
     const double r = (double)acc;  // rounded to nearest
     return acc == 0 ? 0.0 : __hiloint2double(__double2hiint(r) + (int)((top - 2103u) << 20), __double2loint(r));
