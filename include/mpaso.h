@@ -292,14 +292,15 @@ int mpaso_state_device_bytes(mpaso_state s, int64_t *bytes);
  * tracers (the tracer fluxes move from the first kernel into the edge threads
  * of the second, the limiter into a kernel of its own).  Results do not
  * depend on the threads per block, the L2 choice, the launch overlap or the
- * schedule; the other variants may
- * differ in the last bits.  A state reports 256 threads and no overlap until a
- * configuration is set or tuned; until then its launches choose both by the
- * mesh's size.  No counterpart in the reference (its tasks have
- * no device launch shape).  Setting it drops any captured step graph; a
- * persisting L2 reservation is per device context, so at most one state per
- * device should use config[9] != 0, and destroying it releases the
- * reservation. */
+ * schedule; the other variants may differ in the last bits.  The
+ * configuration that a new state reports
+ * (everything unrolled, 256 threads, one lane, all else 0) names the untuned
+ * form: block sizes, launch overlap and, in the sw app without tracers,
+ * fused launches by the mesh's size.  Setting it returns a state to that.
+ * No counterpart in the reference (its tasks have no device launch shape).
+ * Setting a configuration drops any captured step graph; a persisting L2
+ * reservation is per device context, so at most one state per device should
+ * use config[9] != 0, and destroying it releases the reservation. */
 int mpaso_state_launch_config(mpaso_state s, int32_t *config);
 int mpaso_state_set_launch_config(mpaso_state s, const int32_t *config);
 /* The same with n >= 12 ints, the 13th being the threads per edge-level of
@@ -315,9 +316,11 @@ int mpaso_state_set_launch_config_ex(mpaso_state s, const int32_t *config, int32
  * kernel of the sw app 1, 2 or 4 threads per edge-level) over nsteps steps
  * of size dt and keeps the fastest, then picks the L2 residency choice on
  * the whole stage, the schedule on the whole stage and the launch overlap on
- * uninterrupted steps.  The prognostic state is saved first and restored on
- * return, so the call leaves (h, u, tracers) unchanged; it allocates one
- * temporary copy of them.  config (may be NULL) receives the chosen
+ * uninterrupted steps; last, replayed steps of the result against the untuned
+ * form, which stays unless the result is clearly faster.  The prognostic state
+ * is saved first and restored on return, so the call leaves (h, u, tracers)
+ * unchanged; it allocates one temporary copy of them.  If it fails, the state
+ * keeps the configuration it had.  config (may be NULL) receives the chosen
  * configuration (12 ints).  Call it outside stream capture. */
 int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *config);
 

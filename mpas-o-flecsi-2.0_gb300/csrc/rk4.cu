@@ -1137,8 +1137,35 @@ void get_config(const SwState &S, int32_t *config) {
   config[11] = S.tune_split;
 }
 
+// The configuration a state begins with names the launch rules (rk4.cuh), so that
+// it can be read, kept and set again like any other.
+bool names_rules(const SwState &S) {
+  for (int k = 0; k < 3; ++k)
+    if (!S.tune_unroll[k] || S.tune_tpb[k] != 256 || S.tune_occ[k]) return false;
+  return !S.tune_l2 && !S.tune_pdl && !S.tune_split && S.tune_lanes == 1;
+}
+
+// The launch configuration as a value (the autotuner keeps and puts back several).
+struct Tuning {
+  int unroll[3] = {1, 1, 1}, tpb[3] = {256, 256, 256}, occ[3] = {0, 0, 0};
+  int l2 = 0, pdl = 0, split = 0, lanes = 1;
+  bool rules = true;
+  Tuning() = default;
+  explicit Tuning(const SwState &S)
+      : l2(S.tune_l2), pdl(S.tune_pdl), split(S.tune_split), lanes(S.tune_lanes), rules(S.tune_auto) {
+    for (int k = 0; k < 3; ++k) unroll[k] = S.tune_unroll[k], tpb[k] = S.tune_tpb[k], occ[k] = S.tune_occ[k];
+  }
+};
+
 // Whether the state may run its TRiSK loop with several lanes per edge.
 bool has_lanes(const SwState &S) { return S.p.app == MPASO_APP_SW && S.T <= kLanesMaxT; }
+
+void apply(SwState &S, const Tuning &t) {
+  drop_graph(S);
+  for (int k = 0; k < 3; ++k) S.tune_unroll[k] = t.unroll[k], S.tune_tpb[k] = t.tpb[k], S.tune_occ[k] = t.occ[k];
+  S.tune_pdl = t.pdl, S.tune_split = t.split, S.tune_lanes = t.lanes, S.tune_auto = t.rules;
+  set_l2_window(S, t.l2);
+}
 
 constexpr int kTpbChoices[3] = {64, 128, 256};
 
@@ -1685,8 +1712,8 @@ int mpaso_state_set_launch_config(mpaso_state s, const int32_t *config) {
       S.tune_unroll[k] = config[k], S.tune_tpb[k] = config[3 + k], S.tune_occ[k] = config[6 + k];
     set_l2_window(S, config[9]);
     S.tune_pdl = config[10];
-    S.tune_auto = false;
     S.tune_split = S.p.app == MPASO_APP_SW && S.T > 0 ? config[11] : 0;
+    S.tune_auto = names_rules(S);
   });
 }
 
@@ -1709,8 +1736,32 @@ int mpaso_state_set_launch_config_ex(mpaso_state s, const int32_t *config, int32
     const int rc = mpaso_state_set_launch_config(s, config);
     if (rc != MPASO_OK) fail(rc, mpaso_last_error());
     s->s.tune_lanes = lanes;
+    s->s.tune_auto = names_rules(s->s);
   });
 }
+
+namespace {
+// Device time (ms) of a replayed step after one untimed replay; advances the state.
+double time_graph_steps(SwState &S, double dt, int nsteps) {
+  struct Events {
+    cudaEvent_t a = nullptr, b = nullptr;
+    ~Events() {
+      if (a) cudaEventDestroy(a);
+      if (b) cudaEventDestroy(b);
+    }
+  } ev;
+  float ms = 0.f;
+  MPASO_CUDA(cudaEventCreate(&ev.a));
+  MPASO_CUDA(cudaEventCreate(&ev.b));
+  step_graph(S, dt, 1);
+  MPASO_CUDA(cudaEventRecord(ev.a, S.stream));
+  step_graph(S, dt, nsteps);
+  MPASO_CUDA(cudaEventRecord(ev.b, S.stream));
+  MPASO_CUDA(cudaEventSynchronize(ev.b));
+  MPASO_CUDA(cudaEventElapsedTime(&ms, ev.a, ev.b));
+  return ms / nsteps;
+}
+}  // namespace
 
 int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *config) {
   return guarded("mpaso_state_autotune", [&] {
@@ -1738,6 +1789,7 @@ int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *conf
       }
       S.diag_valid = false;
     };
+    const Tuning before(S);
     try {
       drop_graph(S);
       S.tune_auto = false;
@@ -1804,11 +1856,31 @@ int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *conf
         }
         S.tune_pdl = t[0] < 0.98 * t[1] ? 0 : 1;
       }
+      // The launch rules, which fuse launches no configuration names, against what
+      // was found: replayed steps as the caller will run them, the two in turn, the
+      // best of five each.  The rules stay unless the configuration is clearly
+      // faster (level 4 without tracers 31.2 us per step against 37.4; level 6 with
+      // one 111 against 124; level 5 with one 66.1 against 64.0).
+      const Tuning found(S);
+      double t_found = 1e300, t_rules = 1e300;
+      for (int rep = 0; rep < 5; ++rep)
+        for (const bool rules : {false, true}) {
+          apply(S, rules ? Tuning() : found);
+          save_restore(false);
+          double &t = rules ? t_rules : t_found;
+          t = std::min(t, time_graph_steps(S, dt, nsteps));
+        }
+      apply(S, t_found < 0.98 * t_rules ? found : Tuning());
+      S.tune_auto = names_rules(S);
       save_restore(false);
       MPASO_CUDA(cudaStreamSynchronize(S.stream));
     } catch (...) {
       cudaStreamSynchronize(S.stream);
       cudaFree(keep);
+      try {
+        apply(S, before);
+      } catch (...) {  // the first error is the one to report
+      }
       throw;
     }
     MPASO_CUDA(cudaFree(keep));

@@ -180,8 +180,8 @@ struct SwState {
   int tune_unroll[3] = {1, 1, 1};
   int tune_tpb[3] = {256, 256, 256};
   int tune_occ[3] = {0, 0, 0};
-  // until a configuration is set or tuned the launches go by the rules of
-  // stage_tpb() and stage_pdl()
+  // in the configuration that a state begins with, whose values stand for the
+  // rules below, the launches go by stage_tpb(), stage_pdl() and stage_fused()
   bool tune_auto = true;
   // L2 residency of one static array across the step: 0 none, 1 the advection
   // coefficient pairs (read by K1), 2 the TRiSK weights (read by K2); the
