@@ -49,7 +49,7 @@ struct Lev {
   __device__ __forceinline__ void split(int64_t i, int &e, int &k) const {
     const uint64_t q = __umul64hi((uint64_t)i, mul);
     e = L == 1 ? (int)i : (int)q;
-    k = (int)i - e * L;
+    k = (int)((uint32_t)i - (uint32_t)e * (uint32_t)L);  // modulo 2^32, as e L may exceed an int
   }
 };
 

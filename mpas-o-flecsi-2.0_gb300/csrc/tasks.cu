@@ -808,7 +808,6 @@ int mpaso_oc_calc_provisional_layer_thicknesses(mpaso_mesh m, int32_t nlev,
   return guarded("mpaso_oc_calc_provisional_layer_thicknesses", [&] {
     check_levels(nlev, 0);
     TaskIO io(m, stream);
-    require(io.ctx().has_fct || true, MPASO_ERR_ARG, "");
     const int L = nlev;
     const int ih = io.in(layerThickness, MPASO_CELLS, L), intf = io.in(normalThicknessFlux, MPASO_EDGES, L);
     const int op = io.out(hProv, MPASO_CELLS, L), opi = io.out(hProvInv, MPASO_CELLS, L);
