@@ -1858,9 +1858,9 @@ int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *conf
       }
       // The launch rules, which fuse launches no configuration names, against what
       // was found: replayed steps as the caller will run them, the two in turn, the
-      // best of five each.  The rules stay unless the configuration is clearly
-      // faster (level 4 without tracers 31.2 us per step against 37.4; level 6 with
-      // one 111 against 124; level 5 with one 66.1 against 64.0).
+      // best of five each.  The rules stay unless the configuration is 1% faster
+      // (level 4 without tracers 31.2 us per step against 37.4; level 6 with one 111
+      // against 124; level 5 with one 66.1 against 64.0, level 7 347 against 342).
       const Tuning found(S);
       double t_found = 1e300, t_rules = 1e300;
       for (int rep = 0; rep < 5; ++rep)
@@ -1870,7 +1870,7 @@ int mpaso_state_autotune(mpaso_state s, double dt, int32_t nsteps, int32_t *conf
           double &t = rules ? t_rules : t_found;
           t = std::min(t, time_graph_steps(S, dt, nsteps));
         }
-      apply(S, t_found < 0.98 * t_rules ? found : Tuning());
+      apply(S, t_found < 0.99 * t_rules ? found : Tuning());
       S.tune_auto = names_rules(S);
       save_restore(false);
       MPASO_CUDA(cudaStreamSynchronize(S.stream));
