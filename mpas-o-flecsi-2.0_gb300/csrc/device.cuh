@@ -122,7 +122,9 @@ struct MeshCtx {
   // task call; `d` itself where the context keeps the reference's numbering).
   DMesh ref{};
   bool has_ref = false;
-  std::mutex ref_mutex;  // task calls of several threads
+  // builds the view once; a context is one host thread's at a time, so this is only
+  // for callers who keep their streams apart but not their threads
+  std::mutex ref_mutex;
   void *ref_arena = nullptr;
   size_t ref_bytes = 0;
   const DMesh &task_view();

@@ -6,9 +6,11 @@
 // budget), code running under a strict no-cudaMalloc policy because
 // cudaMalloc/cudaFree can synchronize the whole device and stall other work,
 // or a process that has already handed nearly all HBM to a pool.  The regular
-// mpaso_sw_compute_tend stages its arguments through a scratch buffer that the
-// mesh context grows with cudaMalloc on demand; this variant stages them
-// through one fixed array compiled into the library instead.
+// mpaso_sw_compute_tend allocates with cudaMalloc: on a context's first task call
+// a copy of the mesh in the caller's numbering, and for host arrays, or an output
+// that overlaps another argument, a scratch buffer that grows on demand.  This
+// variant runs in the context's own numbering and permutes its arguments through
+// one fixed array compiled into the library instead.
 //
 // The array is a file-scope __device__ buffer of kScratchDoubles doubles
 // (32 MiB).  Every GPU that loads the library holds it until the process

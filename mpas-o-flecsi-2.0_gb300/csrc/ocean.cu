@@ -28,8 +28,8 @@
 //
 // The FP64 pipe bounds these kernels (82-84% busy with every product and sum on
 // it, the issue slots 10-24%), so the products run on the integer pipe
-// (softmul.cuh, the same rounding bit for bit) and only the sums on the FP64
-// pipe.  Level-6 sphere, 60 levels x 3 tracers, us per launch: oc_edges 1384 ->
+// (softmul.cuh, the same rounding; the sign of a zero aside) and only the sums on
+// the FP64 pipe.  Level-6 sphere, 60 levels x 3 tracers, us per launch: oc_edges 1384 ->
 // 630 (FP64, ALU and issue each 62-66% busy), oc_cells 659 -> 399, oc_final 484 ->
 // 356 (451 and 363 with a branch to the hardware product after each slot; their
 // registers are capped at 80 and 64, uncapped 448 and 371).

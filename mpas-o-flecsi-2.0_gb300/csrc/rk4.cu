@@ -118,6 +118,8 @@ __device__ __forceinline__ void tend_item(const DMesh &m, const DStat &st, const
   if (i < nEL * LANES) {
     const int lane = (int)(i & (LANES - 1));
     i /= LANES;
+    // (divided, here and for the cells: Lev::split holds its factor in registers,
+    // level 7 41.3 us per launch against 40.4, 3 levels 86.0 against 84.0)
     const int e = (int)(i / (int)L), k = (int)(i - (int64_t)e * L);
     // q = sum_j W_j F_j (pv_e + pv_j) / 2 = (Pv_e sum W/8 F2_j + sum W/8 F2_j Pv_j)
     double s1 = 0.0, s2 = 0.0;
@@ -333,7 +335,7 @@ __device__ __forceinline__ void vertex_diag(const DMesh &m, const DStat &st, con
 
 // ------------------------------------------------------ K3: cells + vertices
 // SOFT: the cells' squares and tracer products on the integer pipe, bit for bit the
-// same (launch_k3 says when).
+// same but for the sign of a zero (launch_k3 says when).
 template <int T, int NC, bool SOFT = false>
 __device__ __forceinline__ void final_item(const DMesh &m, const DStat &st, const Stage &S, Lev L, int64_t i) {
   const int64_t nCL = (int64_t)m.nC * L;

@@ -97,9 +97,10 @@ struct Stage {
   int fct, hmix, visc, pin_u;
   // sw: the mesh fills the GPU, where the last kernel is bound by the FP64 pipe: the
   // products of the vertex part and (without tracers) the squared velocities go
-  // to the integer pipe, the same values bit for bit, at some hundred cycles of
-  // latency that a smaller mesh would only wait for (level 7, no tracer: 206 -> 197
-  // us per step, one tracer 354 -> 351; level 3 90 -> 92, so not there)
+  // to the integer pipe, the same values (the sign of a zero aside), at some
+  // hundred cycles of latency that a smaller mesh would only wait for (level 7, no
+  // tracer: 206 -> 197 us per step, one tracer 354 -> 351; level 3 90 -> 92, so not
+  // there)
   int fill;
   int centred;          // without FCT: the sw app's centred tracer flux (1) or no advection (0, ocean)
   const double *u_in, *h_in, *tr_in;        // stage input

@@ -6,8 +6,8 @@
 // -fmad=false, so no multiply-add is fused), and scatter loops of the
 // reference become gathers over the reverse connectivity in the order the
 // scatter visited them.  Results therefore agree value for value with the
-// reference tasks (bit for bit, signs of zero in the ocean tasks aside).  One
-// thread per (entity, level); tracers loop inside.
+// reference tasks (bit for bit, signs of zero in the ocean tasks aside), infinities
+// and NaN included.  One thread per (entity, level); tracers loop inside.
 #include <type_traits>
 
 #include "softmul.cuh"
@@ -185,8 +185,8 @@ __global__ void k_oc_ntf(int64_t n, const double *hE, const double *u, double *n
 // leaves the FP64 pipe the sums; tracers are unrolled at compile time, and what
 // levels share (1 / area, the mixing coefficient) is not divided out in each.
 // Level 5, 20 levels x 3 tracers, us: high order 130 -> 63, fct_a + fct_b + fct_c
-// 187 -> 83, hmix 128 -> 36, accumulate 35 -> 20, low order 20 -> 11, provisional
-// 20 -> 16; a tracer stage task by task 456 -> 184.
+// 187 -> 87, hmix 128 -> 34, accumulate 35 -> 21, low order 20 -> 11, provisional
+// 20 -> 16; a tracer stage task by task 456 -> 186.
 
 // IEEE a < b on the integer pipe (false with a NaN; zeros are equal).
 __device__ __forceinline__ bool ieee_lt(double a, double b) {
